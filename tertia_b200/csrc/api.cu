@@ -544,6 +544,7 @@ struct Engine : EngineBase {
                                                 "in [32, 1024]");
             if ((s = alloc(&scratch2, 6 * plane, "transform scratch"))) return s;
         }
+        if (!tcx && !fftx && !fftx64) CK(dtt_dense_setup<T>());
         if (sizeof(T) == 8 && getenv("QS_FP32_STUDY")) {
             fp32_study = atoi(getenv("QS_FP32_STUDY")) & 1023;
             if (fp32_study & 1) {

@@ -152,6 +152,11 @@ extern "C" qs_status qs_transform2d_noalloc(int kind_z, int kind_y, int ny, int 
     qs_status s = scratch_on_current_device(&scratch);
     if (s) return s;
     cudaStream_t st = (cudaStream_t)stream;
+    {   // every call: the context may be another one than the last call's
+        const cudaError_t e = dtt_dense_setup<double>();
+        if (e != cudaSuccess)
+            return fail(QS_ERR_CUDA, std::string("transform set-up: ") + cudaGetErrorString(e));
+    }
     const size_t plane = (size_t)ny * nz;
     double* mat_y = scratch;
     double* mat_z = mat_y + (size_t)ny * ny;

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs<T> a) {
 #pragma unroll
     for (int c = 0; c < NV; c++) v[c] = T(0);
 
+    pdl_wait();
     if (i < a.n) {
         const T one = T(1), two = T(2), half = T(0.5);
         const int cell = a.cell[i];
@@ -351,6 +352,7 @@ __global__ void __launch_bounds__(256) push_kernel(PushArgs<T> a) {
         }
     }
 
+    pdl_trigger();
     // warp-segmented sum over runs of equal first-deposit cell
     const unsigned full = 0xffffffffu;
     const int nextKey = __shfl_down_sync(full, key, 1);
@@ -869,10 +871,10 @@ int launch_push(const PushArgs<T>& a, int shape, bool precise, cudaStream_t st) 
                 launch_pdl(push_cell_kernel<4>, dim3((cells + 127) / 128), dim3(128), 0, st, a);
                 return 1;
             }
-            push_kernel<T, QS_SHAPE_NGP, true, true><<<blocks, threads, 0, st>>>(a);
+            launch_pdl(push_kernel<T, QS_SHAPE_NGP, true, true>, dim3(blocks), dim3(threads), 0, st, a);
         } else {
-            if (precise) push_kernel<T, QS_SHAPE_NGP, true, false><<<blocks, threads, 0, st>>>(a);
-            else push_kernel<T, QS_SHAPE_NGP, false, false><<<blocks, threads, 0, st>>>(a);
+            if (precise) launch_pdl(push_kernel<T, QS_SHAPE_NGP, true, false>, dim3(blocks), dim3(threads), 0, st, a);
+            else launch_pdl(push_kernel<T, QS_SHAPE_NGP, false, false>, dim3(blocks), dim3(threads), 0, st, a);
         }
     } else {
         if constexpr (F32) {
@@ -880,7 +882,7 @@ int launch_push(const PushArgs<T>& a, int shape, bool precise, cudaStream_t st) 
         } else {
             if (a.loff && !a.dep_cell) return launch_push_rows_f64(a, st);
         }
-        push_kernel<T, QS_SHAPE_CIC, true, F32><<<blocks, threads, 0, st>>>(a);
+        launch_pdl(push_kernel<T, QS_SHAPE_CIC, true, F32>, dim3(blocks), dim3(threads), 0, st, a);
     }
     return 1;
 }

@@ -106,7 +106,10 @@ int launch_add_increment(double* dst, const float* now, const float* before, siz
 template <class T>
 int launch_convert_back(const T* src, double* dst, size_t n, cudaStream_t st);
 
-// Transforms.
+// Transforms.  dtt_dense_setup: the dense pass kernel's opt-in to its dynamic
+// shared memory, on the current device, before its first launch there.
+template <class T>
+cudaError_t dtt_dense_setup();
 template <class T>
 int run_dtt_simt(const DttJob<T>& job, int ny, int nz, const DttMats<T>& my,
                  const DttMats<T>& mz, T* scratch, cudaStream_t st);

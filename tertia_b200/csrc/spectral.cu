@@ -19,6 +19,7 @@
 #include "split.cuh"
 #include "density.cuh"
 #include "charge.cuh"
+#include "pdl.cuh"
 
 namespace qs {
 
@@ -40,6 +41,8 @@ template <class T>
 __global__ void predictor_kernel(SpecArgs<T> a) {
     const int n1 = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = a.ny * a.nz;
+    pdl_wait();
+    pdl_trigger();
     if (n1 >= N) return;
     const int j = n1 % a.ny, k = n1 / a.ny;
     const T d = *a.dens_p, hx = a.hx;
@@ -94,6 +97,8 @@ __global__ void corrector_kernel(SpecArgs<T> a) {
     const int n1 = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = a.ny * a.nz;
     double qr = 0.0, qj = 0.0;
+    pdl_wait();
+    pdl_trigger();
     if (n1 < N) corrector_mode(a, n1, qr, qj);
     if (a.qsum) charge_block_sum(qr, qj, a.qsum + 2 * (size_t)blockIdx.x);
 }
@@ -153,7 +158,7 @@ int launch_predictor(const SpecArgs<T>& a, cudaStream_t st) {
         if (launch_predictor_fast(a, st)) return 1;
     }
     const int N = a.ny * a.nz;
-    predictor_kernel<T><<<(N + 255) / 256, 256, 0, st>>>(a);
+    launch_pdl(predictor_kernel<T>, dim3((N + 255) / 256), dim3(256), 0, st, a);
     return 1;
 }
 template <class T>
@@ -162,7 +167,7 @@ int launch_corrector(const SpecArgs<T>& a, cudaStream_t st) {
         if (launch_corrector_fast(a, st)) return 1;
     }
     const int N = a.ny * a.nz;
-    corrector_kernel<T><<<(N + 255) / 256, 256, 0, st>>>(a);
+    launch_pdl(corrector_kernel<T>, dim3((N + 255) / 256), dim3(256), 0, st, a);
     return 1;
 }
 
