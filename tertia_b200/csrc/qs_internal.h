@@ -61,7 +61,7 @@ template <class T>
 int launch_beam_check(const T* b3, int nlayers, size_t plane, int* err, double* part,
                       cudaStream_t st);
 // out[layer * 2 + q] = scale * sum over p < nparts of part[2 * (layer * nparts + p) + q]
-// (q = 0, 1; in index order)
+// (q = 0, 1; in a fixed order)
 int launch_charge_reduce(const double* part, int nparts, int nlayers, double scale, double* out,
                          cudaStream_t st);
 
