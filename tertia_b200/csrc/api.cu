@@ -644,6 +644,7 @@ struct Engine : EngineBase {
             a.hxhy = (float)((cfg.hx / S) / cfg.hy);
             a.hxhz = (float)((cfg.hx / S) / cfg.hz);
             a.invMy = 1.0f / (float)My;
+            a.lgMy = lg_my();
             a.full = full;
             a.err = d_err;
             float* before = study_p + 6 * (size_t)np_cap;   // the float state before the push
@@ -711,6 +712,14 @@ struct Engine : EngineBase {
         }
         j.scale = scale;
         return j;
+    }
+
+    // log2 My when both transverse sizes are powers of two, else -1
+    int lg_my() const {
+        if ((My & (My - 1)) || (Mz & (Mz - 1))) return -1;
+        int l = 0;
+        while ((1 << l) < My) l++;
+        return l;
     }
 
     T inv_scale() const { return (T)(1.0 / (4.0 * (double)My * (double)Mz)); }
@@ -1487,6 +1496,7 @@ struct Engine : EngineBase {
         a.hxhy = (T)((cfg.hx / S) / cfg.hy);
         a.hxhz = (T)((cfg.hx / S) / cfg.hz);
         a.invMy = 1.0f / (float)My;
+        a.lgMy = lg_my();
         // lattice order (particle p seeded in cell p / ppc): the NGP
         // one-thread-per-cell kernel relies on it
         a.uniform_ppc = uniform_layout ? cfg.ppc : 0;

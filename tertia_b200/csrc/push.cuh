@@ -517,17 +517,25 @@ __global__ void __launch_bounds__(128) push_cell_kernel(PushArgs<float> a) {
 //    another cell (it moved since the last regrouping) is added by global
 //    atomics instead; on a full push followed by a regrouping the lane counts
 //    the particles that stay in its cell and adds one count per cell.
-// No shuffles or matches sum the deposits.  The window's slots carry one pad
-// word per 32, so that lanes reading slots about ppc apart hit distinct
-// banks.  At the end each lane spreads its cell's corner sums (the right-hand
-// corners through a shuffle to the next lane), the warps combine their rows
-// in the block tile in two ordered phases, and the tile is flushed with one
-// global atomic per touched cell and current.  Particles gathered outside
-// the tile (moved since the regrouping) read the fields from global memory.
-// ND = 3 leaves out the density deposit, which the march does not read.  The
-// full push stores the particles in place with their new cell.  Same physics
+// No shuffles or matches sum the deposits.  At the end each lane spreads its
+// cell's corner sums (the right-hand corners through a shuffle to the next
+// lane), the warps combine their rows in the block tile in two ordered phases,
+// and the tile is flushed, times the species' charge factors, with one global
+// atomic per touched cell and current.  Particles gathered outside the tile
+// (moved since the regrouping) read the fields from global memory.  ND = 3
+// leaves out the density deposit, which the march does not read.  The full
+// push stores the particles in place with their new cell.  Same physics
 // as push_kernel<T, CIC, precise, fast> (movepart_layer_CIC.cpp:165-193,
 // 449-496 weights), the divisions factored into reciprocals.
+//
+// What bounds it: instruction issue (a half push of 1,048,576 particles at
+// 512 x 512 issues 13.6 M warp instructions, two thirds of the issue slots)
+// and the dependent loads at a block's start.  Against the form with floor(),
+// divided cell indices, unshared 1 + p^2 and one staged word per value
+// (15.1 M instructions, 64 registers): 103.8 -> 98.3 us per layer of the warm
+// 512 x 512 x 1024 march, 407 -> 398 us at 1024 x 1024, 190.7 -> 186.3 us in
+// FP64.  72 registers, 7 blocks per SM; capped at 64 registers the spills cost
+// more than the eighth block gives (105.0 us).
 template <class T>
 __device__ __forceinline__ int cell_offset(const PushArgs<T>& a, int c) {
     return a.loff[c] + a.bpref[c >> 10];
@@ -538,14 +546,16 @@ template <class T>
 struct RowMath;
 template <>
 struct RowMath<float> {
-    static __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
+    static __device__ __forceinline__ float rsq(float x) { return rsq_approx(x); }
     static __device__ __forceinline__ float rcp(float x) { return rcp_approx(x); }
+    static __device__ __forceinline__ float twice_rcp(float x) { return 2.f * rcp_approx(x); }
     static __device__ __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
 };
 template <>
 struct RowMath<double> {
     static __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
     static __device__ __forceinline__ double rcp(double x) { return 1.0 / x; }
+    static __device__ __forceinline__ double twice_rcp(double x) { return 2.0 / x; }
     static __device__ __forceinline__ double div(double a, double b) { return a / b; }
 };
 
@@ -571,20 +581,99 @@ __device__ __forceinline__ void cic_substep(T dy, T dz, T ps, T& ytmp, T& ztmp, 
     wc[3] = ry * rz;
 }
 
-template <int TY, int ND, int WIN, class T>
+// (j, k) of a cell, and an index wrapped into its period: bit operations when
+// the sizes are powers of two (P2), else the general forms
+template <bool P2, class T>
+__device__ __forceinline__ void split_cell(const PushArgs<T>& a, int cell, int& j, int& k) {
+    if constexpr (P2) {
+        j = cell & (a.My - 1);
+        k = cell >> a.lgMy;
+    } else {
+        cell_jk(cell, a.My, a.invMy, j, k);
+    }
+}
+template <bool P2>
+__device__ __forceinline__ int wrap_p(int j, int M) {
+    if constexpr (P2) return j & (M - 1);
+    else return wrap1(j, M);
+}
+
+// One axis of a move by d, |d| <= 1, from y in [0, 1]: the in-cell position
+// and the cell shift.  u = y + d lies in [-1, 2], so that floor(u) is two
+// comparisons (floor and the conversion to int run at a quarter of their
+// rate); a position that rounds to 1 belongs to the next cell.
+template <class T>
+__device__ __forceinline__ T move_axis(T y, T d, int& s) {
+    const T u = y + d;
+    const bool up = u >= T(1), dn = u < T(0);
+    T r = up ? u - T(1) : u;
+    r = dn ? u + T(1) : r;
+    s = (up ? 1 : 0) - (dn ? 1 : 0);
+    if (r >= T(1)) {
+        r = T(0);
+        s += 1;
+    }
+    return r;
+}
+
+// The deposits staged between the two phases of the grouped push, one slot
+// per particle of a warp's window: the charges q, the in-cell position and the
+// cell of the first sub-step.  In FP32 without the density two vector words,
+// so that a slot costs two stores and two loads instead of six; lanes of
+// phase 2 read slots about ppc apart, and one pad word per 8 slots of 16
+// bytes (per 16 slots of 8 bytes) puts these on distinct banks.  The other
+// variants keep one array per value, with one pad per 32 slots.
+template <class T, int ND, int WIN>
+struct DepositStage {
+    T v[ND + 2][WIN + WIN / 32];
+    int key[WIN + WIN / 32];
+    __device__ __forceinline__ void put(int s, const T (&q)[ND], T ry, T rz, int k) {
+        const int p = s + (s >> 5);
+#pragma unroll
+        for (int d = 0; d < ND; d++) v[d][p] = q[d];
+        v[ND][p] = ry;
+        v[ND + 1][p] = rz;
+        key[p] = k;
+    }
+    __device__ __forceinline__ int get(int s, T (&q)[ND], T& ry, T& rz) const {
+        const int p = s + (s >> 5);
+#pragma unroll
+        for (int d = 0; d < ND; d++) q[d] = v[d][p];
+        ry = v[ND][p];
+        rz = v[ND + 1][p];
+        return key[p];
+    }
+};
+template <int WIN>
+struct DepositStage<float, 3, WIN> {
+    float4 a[WIN + WIN / 8];
+    float2 b[WIN + WIN / 16];
+    __device__ __forceinline__ void put(int s, const float (&q)[3], float ry, float rz, int k) {
+        a[s + (s >> 3)] = make_float4(q[0], q[1], q[2], ry);
+        b[s + (s >> 4)] = make_float2(rz, __int_as_float(k));
+    }
+    __device__ __forceinline__ int get(int s, float (&q)[3], float& ry, float& rz) const {
+        const float4 x = a[s + (s >> 3)];
+        const float2 y = b[s + (s >> 4)];
+        q[0] = x.x; q[1] = x.y; q[2] = x.z;
+        ry = x.w;
+        rz = y.x;
+        return __float_as_int(y.y);
+    }
+};
+
+template <int TY, int ND, int WIN, bool P2, class T>
 __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     using M = RowMath<T>;
     using FP = FPair<T>;
-    using P2 = typename FP::type;
+    using P2T = typename FP::type;
     constexpr int TX = 32, W = TX + 1, H = TY + 1;
-    constexpr int NS = ND + 2;           // staged per slot: ND charges, in-cell y and z
-    constexpr int WP = WIN + WIN / 32;   // one pad word per 32 slots
     static_assert(WIN % 32 == 0, "whole warps per window");
     const T one = T(1), zero = T(0), half = T(0.5);
-    __shared__ P2 Fs[3][H][W];           // field pairs of the tile cells + one row/column (P, C averaged)
+    __shared__ P2T Fs[3][H][W];          // field pairs of the tile cells + one row/column (P, C averaged)
     __shared__ T Tt[ND][H][W];           // block deposit tile [current][row][col]
-    __shared__ T S[TY][NS][WP];          // staged deposits of the window
-    __shared__ int K[TY][2][WP];         // [0]: first sub-step's cell (-1: none); [1]: final cell
+    __shared__ DepositStage<T, ND, WIN> S[TY];   // staged deposits of each warp's window
+    __shared__ int Kl[TY][WIN + WIN / 32];       // counting push: the final cells
     const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
     const int My = a.My, Mz = a.Mz;
     const size_t plane = a.plane;
@@ -594,14 +683,24 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     QS_TRACE_ENTRY();
     pdl_wait();
     QS_TRACE_WAITED();
+    const bool one_set = a.P == a.C;     // an averaged set: (x + x) / 2 = x
     for (int i = threadIdx.x; i < H * W; i += 32 * TY) {
         const int r = i / W, cc = i - r * W;
-        const size_t m = (size_t)wrap1(j0 + cc, My) + (size_t)My * wrap1(k0 + r, Mz);
+        const size_t m = (size_t)wrap_p<P2>(j0 + cc, My) + (size_t)My * wrap_p<P2>(k0 + r, Mz);
+        if (one_set) {
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const P2 pp = FP::make(ld(a.P + 2 * q * plane + m), ld(a.P + (2 * q + 1) * plane + m));
-            const P2 cp = FP::make(ld(a.C + 2 * q * plane + m), ld(a.C + (2 * q + 1) * plane + m));
-            Fs[q][r][cc] = FP::mul(half, FP::add(pp, cp));
+            for (int q = 0; q < 3; q++)
+                Fs[q][r][cc] =
+                    FP::make(ld(a.C + 2 * q * plane + m), ld(a.C + (2 * q + 1) * plane + m));
+        } else {
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                const P2T pp =
+                    FP::make(ld(a.P + 2 * q * plane + m), ld(a.P + (2 * q + 1) * plane + m));
+                const P2T cp =
+                    FP::make(ld(a.C + 2 * q * plane + m), ld(a.C + (2 * q + 1) * plane + m));
+                Fs[q][r][cc] = FP::mul(half, FP::add(pp, cp));
+            }
         }
     }
     __syncthreads();
@@ -626,10 +725,23 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     const int pend = __shfl_sync(0xffffffffu, hi, 31);
     const bool count = a.full && a.cnt;
     int stay = 0;                        // particles that end the full push in mycell
-    // the cell's sums of current d at its corners (0, 1) and (2, 3)
-    P2 acc[ND][2];
+    const T dj[4] = {a.djx0, a.djy0, a.djz0, a.drho0};   // the species' factor of each current
+    // the cell's sums of current d (without dj) at its corners (0, 1) and (2, 3)
+    P2T acc[ND][2];
 #pragma unroll
     for (int d = 0; d < ND; d++) acc[d][0] = acc[d][1] = FP::make(zero, zero);
+    // the 4 corners of cell (jc, kc) get q[d] * dj[d] * weight by global atomics
+    auto scatter = [&](int jc, int kc, const T (&q)[ND], const T (&wc)[4]) {
+        const int jc1 = wrap_p<P2>(jc + 1, My), kc1 = wrap_p<P2>(kc + 1, Mz);
+        const size_t nd[4] = {(size_t)jc + (size_t)My * kc, (size_t)jc1 + (size_t)My * kc,
+                              (size_t)jc + (size_t)My * kc1, (size_t)jc1 + (size_t)My * kc1};
+#pragma unroll
+        for (int d = 0; d < ND; d++) {
+            const T x = q[d] * dj[d];
+#pragma unroll
+            for (int r = 0; r < 4; r++) atomicAdd(a.dep + d * plane + nd[r], x * wc[r]);
+        }
+    };
     // the particle of the next pass is loaded while this one is pushed
     int nx_cell = 0;
     T nx_y = zero, nx_z = zero, nx_px = zero, nx_py = zero, nx_pz = zero, nx_w = zero;
@@ -660,15 +772,15 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                     atomicOr(a.err, DEV_ERR_RANGE);   // no deposit; it stays in its cell
                 } else {
                     int j, k;
-                    cell_jk(cell, My, a.invMy, j, k);
+                    split_cell<P2>(a, cell, j, k);
                     const T wg[4] = {(one - yp) * (one - zp), yp * (one - zp), (one - yp) * zp,
                                      yp * zp};
                     T g[6];
                     const int tj = j - j0, tk = k - k0;
-                    if (tj >= 0 && tj < TX && tk >= 0 && tk < TY) {
+                    if ((unsigned)tj < TX && (unsigned)tk < TY) {
 #pragma unroll
                         for (int q = 0; q < 3; q++) {
-                            P2 gq = FP::mul(wg[0], Fs[q][tk][tj]);
+                            P2T gq = FP::mul(wg[0], Fs[q][tk][tj]);
                             gq = FP::fma(wg[1], Fs[q][tk][tj + 1], gq);
                             gq = FP::fma(wg[2], Fs[q][tk + 1][tj], gq);
                             gq = FP::fma(wg[3], Fs[q][tk + 1][tj + 1], gq);
@@ -676,7 +788,7 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                             g[2 * q + 1] = gq.y;
                         }
                     } else {
-                        const int j1 = wrap1(j + 1, My), k1 = wrap1(k + 1, Mz);
+                        const int j1 = wrap_p<P2>(j + 1, My), k1 = wrap_p<P2>(k + 1, Mz);
                         const size_t nn[4] = {(size_t)j + (size_t)My * k,
                                               (size_t)j1 + (size_t)My * k,
                                               (size_t)j + (size_t)My * k1,
@@ -691,61 +803,65 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                             g[f] = s;
                         }
                     }
-                    const T inv_gp = M::rsq(one + px * px + py * py + pz * pz);
+                    T inv_gp, omp;                            // 1 - Vx before the kick
+                    vel_terms(px, py, pz, inv_gp, omp);
                     const T Vyp = py * inv_gp, Vzp = pz * inv_gp;
-                    const T omp = one_minus_vx(px, py, pz, inv_gp);   // 1 - Vx before the kick
                     const T kE = a.sE * M::rcp(omp);
                     const T ex = g[0] * kE, ey = g[1] * kE, ez = g[2] * kE;
                     px += ex; py += ey; pz += ez;
                     const T kB = M::rsq(one + px * px + py * py + pz * pz) * kE;
                     const T bx = (g[3] + a.bxe) * kB, by = (g[4] + a.bye) * kB,
                             bz = (g[5] + a.bze) * kB;
-                    const T co = M::div(T(2), one + bx * bx + by * by + bz * bz);
+                    const T co = M::twice_rcp(one + bx * bx + by * by + bz * bz);
                     const T p3x = (py * bz - pz * by + px) * co;
                     const T p3y = (pz * bx - px * bz + py) * co;
                     const T p3z = (px * by - py * bx + pz) * co;
                     px += ex + (p3y * bz - p3z * by);
                     py += ey + (p3z * bx - p3x * bz);
                     pz += ez + (p3x * by - p3y * bx);
-                    const T inv_g = M::rsq(one + px * px + py * py + pz * pz);
+                    T inv_g, omm;
+                    vel_terms(px, py, pz, inv_g, omm);
                     const T Vxm = px * inv_g, Vym = py * inv_g, Vzm = pz * inv_g;
-                    const T Vy = half * (Vym + Vyp), Vz = half * (Vzm + Vzp);
-                    const T inv2 = M::rcp(half * (one_minus_vx(px, py, pz, inv_g) + omp));
+                    const T inv2 = M::rcp(half * (omm + omp));
+                    const T hinv = half * inv2;
                     const T wq = w * inv2;
-                    const T dq[4] = {wq * a.djx0 * Vxm, wq * a.djy0 * Vym, wq * a.djz0 * Vzm,
-                                     wq * a.drho0};
-                    const T dy = Vy * a.hxhy * inv2, dz = Vz * a.hxhz * inv2;
+                    T dy = (Vym + Vyp) * (a.hxhy * hinv), dz = (Vzm + Vzp) * (a.hxhz * hinv);
                     // sub-steps of at most one cell: the first covers 1/step of
                     // the move, partdx what remains of it after the first
                     const T ady = fabs_t(dy), adz = fabs_t(dz);
                     const T mx = ady > adz ? ady : adz;
-                    T partdx = zero, step = one, ps = one;
-                    if (mx > one) { step = mx; partdx = mx - one; ps = M::rcp(step); }
-                    T ytmp = yp, ztmp = zp;
-                    int jb = j, kb = k;
+                    T partdx = zero, step = one, wf = wq;
+                    T dy1 = dy, dz1 = dz;
+                    if (mx > one) {
+                        step = mx;
+                        partdx = mx - one;
+                        const T ps = M::rcp(step);
+                        wf = wq * ps;
+                        // the larger share may round to a little over one cell
+                        dy1 = min(max(dy * ps, -one), one);
+                        dz1 = min(max(dz * ps, -one), one);
+                    }
                     // first sub-step: staged for the cell-parallel sum
-                    T wc[4];
-                    cic_substep<T>(dy, dz, ps, ytmp, ztmp, jb, kb, My, Mz, wc);
+                    int sy, sz;
+                    ay = move_axis(yp, dy1, sy);
+                    az = move_axis(zp, dz1, sz);
+                    int jb = wrap_p<P2>(j + sy, My), kb = wrap_p<P2>(k + sz, Mz);
                     key = jb + My * kb;
-#pragma unroll
-                    for (int d = 0; d < ND; d++) qv[d] = dq[d] * ps;
-                    ay = ytmp;
-                    az = ztmp;
+                    qv[0] = wf * Vxm;
+                    qv[1] = wf * Vym;
+                    qv[2] = wf * Vzm;
+                    if constexpr (ND == 4) qv[3] = wf;
+                    T ytmp = ay, ztmp = az;
                     // further sub-steps: direct atomics
                     while (partdx > zero) {
+                        T ps;
                         if (partdx > one) { partdx -= one; ps = M::rcp(step); }
                         else { ps = M::div(partdx, step); partdx = zero; }
+                        T wc[4];
                         cic_substep<T>(dy, dz, ps, ytmp, ztmp, jb, kb, My, Mz, wc);
-                        const int jb1 = wrap1(jb + 1, My), kb1 = wrap1(kb + 1, Mz);
-                        const size_t nd[4] = {(size_t)jb + (size_t)My * kb,
-                                              (size_t)jb1 + (size_t)My * kb,
-                                              (size_t)jb + (size_t)My * kb1,
-                                              (size_t)jb1 + (size_t)My * kb1};
-#pragma unroll
-                        for (int r = 0; r < 4; r++)
-#pragma unroll
-                            for (int d = 0; d < ND; d++)
-                                atomicAdd(a.dep + d * plane + nd[r], dq[d] * ps * wc[r]);
+                        T qs[ND] = {wq * ps * Vxm, wq * ps * Vym, wq * ps * Vzm};
+                        if constexpr (ND == 4) qs[3] = wq * ps;
+                        scatter(jb, kb, qs, wc);
                     }
                     last = jb + My * kb;
                     if (a.full) {
@@ -754,52 +870,52 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                     }
                 }
             }
-            const int s = base - wbase + lane, sp = s + (s >> 5);
-            K[wr][0][sp] = key;
-            if (count) K[wr][1][sp] = last;
-#pragma unroll
-            for (int d = 0; d < ND; d++) S[wr][d][sp] = qv[d];
-            S[wr][ND][sp] = ay;
-            S[wr][ND + 1][sp] = az;
+            const int s = base - wbase + lane;
+            S[wr].put(s, qv, ay, az, key);
+            if (count) Kl[wr][s + (s >> 5)] = last;
         }
         __syncwarp();
-        // phase 2: lane = cell
+        // phase 2: lane = cell.  Particles that left the cell are noted and
+        // added by global atomics in a loop of their own, which runs as often
+        // as the lane with the most of them needs, not in every pass where
+        // one lane has one.
         const int qa = max(lo, wbase), qb = min(hi, wend);
+        unsigned moved = 0;
+        auto add_moved = [&](int s) {
+            T qv[ND], ry, rz;
+            const int key = S[wr].get(s, qv, ry, rz);
+            const T wc[4] = {(one - ry) * (one - rz), ry * (one - rz), (one - ry) * rz, ry * rz};
+            int kj, kk;
+            split_cell<P2>(a, key, kj, kk);
+            scatter(kj, kk, qv, wc);
+        };
         for (int q = qa; q < qb; q++) {
-            const int s = q - wbase, sp = s + (s >> 5);
-            const int key = K[wr][0][sp];
+            const int s = q - wbase;
+            T qv[ND], ry, rz;
+            const int key = S[wr].get(s, qv, ry, rz);
             if (count) {
-                const int last = K[wr][1][sp];
+                const int last = Kl[wr][s + (s >> 5)];
                 if (last == mycell) stay++;
                 else atomicAdd(a.cnt + last, 1);
             }
-            if (key < 0) continue;
-            const T ry = S[wr][ND][sp], rz = S[wr][ND + 1][sp];
-            T qv[ND];
-#pragma unroll
-            for (int d = 0; d < ND; d++) qv[d] = S[wr][d][sp];
             if (key == mycell) {
                 // corner weights in pairs: (1 - rz) (1 - ry, ry) and rz (1 - ry, ry)
-                const P2 wy = FP::make(one - ry, ry);
-                const P2 w01 = FP::mul(one - rz, wy), w23 = FP::mul(rz, wy);
+                const P2T wy = FP::make(one - ry, ry);
+                const P2T w01 = FP::mul(one - rz, wy), w23 = FP::mul(rz, wy);
 #pragma unroll
                 for (int d = 0; d < ND; d++) {
                     acc[d][0] = FP::fma(qv[d], w01, acc[d][0]);
                     acc[d][1] = FP::fma(qv[d], w23, acc[d][1]);
                 }
-            } else {
-                const T wc[4] = {(one - ry) * (one - rz), ry * (one - rz), (one - ry) * rz,
-                                 ry * rz};
-                int kj, kk;
-                cell_jk(key, My, a.invMy, kj, kk);
-                const int kj1 = wrap1(kj + 1, My), kk1 = wrap1(kk + 1, Mz);
-                const size_t nd[4] = {(size_t)kj + (size_t)My * kk, (size_t)kj1 + (size_t)My * kk,
-                                      (size_t)kj + (size_t)My * kk1, (size_t)kj1 + (size_t)My * kk1};
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int d = 0; d < ND; d++) atomicAdd(a.dep + d * plane + nd[r], qv[d] * wc[r]);
+            } else if (key >= 0) {
+                if (q - qa < 32) moved |= 1u << (q - qa);
+                else add_moved(s);
             }
+        }
+        while (moved) {
+            const int b = __ffs(moved) - 1;
+            moved &= moved - 1;
+            add_moved(qa + b - wbase);
         }
         __syncwarp();
     }
@@ -833,11 +949,11 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     __syncthreads();
     for (int i = threadIdx.x; i < H * W; i += 32 * TY) {
         const int r = i / W, cc = i - r * W;
-        const size_t m = (size_t)wrap1(j0 + cc, My) + (size_t)My * wrap1(k0 + r, Mz);
+        const size_t m = (size_t)wrap_p<P2>(j0 + cc, My) + (size_t)My * wrap_p<P2>(k0 + r, Mz);
 #pragma unroll
         for (int d = 0; d < ND; d++) {
             const T x = Tt[d][r][cc];
-            if (x != zero) atomicAdd(a.dep + d * plane + m, x);
+            if (x != zero) atomicAdd(a.dep + d * plane + m, dj[d] * x);
         }
     }
     QS_TRACE_END(a.full ? trace::K_PUSH_FULL : trace::K_PUSH_HALF);
@@ -849,10 +965,14 @@ int launch_push_rows(const PushArgs<T>& a, cudaStream_t st) {
     constexpr int TY = 4, WIN = 128;
     if (!a.loff || a.dep_cell) return 0;   // grouped by cell with offsets (the engine checks the shape)
     const dim3 grid((a.My / 32) * (a.Mz / TY));
-    if (a.skip_dens)
-        launch_pdl(push_cic_row_kernel<TY, 3, WIN, T>, grid, dim3(32 * TY), 0, st, a);
-    else
-        launch_pdl(push_cic_row_kernel<TY, 4, WIN, T>, grid, dim3(32 * TY), 0, st, a);
+    const dim3 block(32 * TY);
+    if (a.skip_dens) {
+        if (a.lgMy >= 0) launch_pdl(push_cic_row_kernel<TY, 3, WIN, true, T>, grid, block, 0, st, a);
+        else launch_pdl(push_cic_row_kernel<TY, 3, WIN, false, T>, grid, block, 0, st, a);
+    } else {
+        if (a.lgMy >= 0) launch_pdl(push_cic_row_kernel<TY, 4, WIN, true, T>, grid, block, 0, st, a);
+        else launch_pdl(push_cic_row_kernel<TY, 4, WIN, false, T>, grid, block, 0, st, a);
+    }
     return 1;
 }
 

@@ -45,6 +45,36 @@ __device__ __forceinline__ double one_minus_vx(double px, double py, double pz, 
     return px > 0.0 ? fwd : bwd;
 }
 
+// Approximate reciprocal square root: PTX rsqrt.approx.ftz.f32, the same
+// instruction rsqrtf uses without the rescaling of subnormal arguments (the
+// arguments here are 1 + p^2).
+__device__ __forceinline__ float rsq_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// 1 / gamma and 1 - Vx of a momentum together, sharing 1 + p^2 and
+// 1 + py^2 + pz^2: the form above with g (g + px) = 1 + p^2 + g px
+__device__ __forceinline__ void vel_terms(float px, float py, float pz, float& inv_g,
+                                          float& omp) {
+    const float q = fmaf(py, py, fmaf(pz, pz, 1.f));
+    const float s = fmaf(px, px, q);
+    inv_g = rsq_approx(s);
+    const float fwd = q * rcp_approx(fmaf(s * inv_g, px, s));
+    const float bwd = fmaf(-px, inv_g, 1.f);
+    omp = px > 0.f ? fwd : bwd;
+}
+__device__ __forceinline__ void vel_terms(double px, double py, double pz, double& inv_g,
+                                          double& omp) {
+    const double q = fma(py, py, fma(pz, pz, 1.0));
+    const double s = fma(px, px, q);
+    inv_g = rsqrt(s);
+    const double fwd = q / fma(s * inv_g, px, s);
+    const double bwd = fma(-px, inv_g, 1.0);
+    omp = px > 0.0 ? fwd : bwd;
+}
+
 // j within one period of [0, M) (a shift of at most one period): no loop
 __device__ __forceinline__ int wrap1(int j, int M) {
     j += (j < 0) ? M : 0;

@@ -65,6 +65,7 @@ struct PushArgs {
     T hx, hy, hz, q2m, djx0, djy0, djz0, drho0, bxe, bye, bze;
     T sE, hxhy, hxhz;     // q2m*hx/2, hx/hy, hx/hz (factored FP32 form)
     float invMy;          // 1/My for the cell index split
+    int lgMy;             // log2 My when My and Mz are powers of two, else -1
     int uniform_ppc;      // >0: particle p sits in cell p / uniform_ppc (lattice layout)
     // FP32 CIC over particles grouped by cell: cell c holds particles
     // loff[c] + bpref[c / 1024] .. (next cell's offset) - 1; the full push
