@@ -1468,7 +1468,9 @@ struct Engine : EngineBase {
         // ClearCurrentsSplit: inside the march the preceding spectral kernel
         // already cleared Csrc
         if (!clear_by_maps()) CK(cudaMemsetAsync(Csrc, 0, 4 * plane * sizeof(T), st));
+        bool as_grouped = true;   // this call changes neither the particles nor their offsets first
         if (cic_sort) {
+            as_grouped = grp.grouped && grp.off_valid;
             qs_status s = cic_prepare();
             if (s) return s;
         }
@@ -1509,6 +1511,9 @@ struct Engine : EngineBase {
         if (cic_sort) {
             a.loff = cic_loff;
             a.bpref = cic_bpref;
+            // in the march a z-pass (every thread of which waits for the
+            // kernel before it) stands between two pushes
+            a.early = (g_pdl && in_march && !adj_recompute && fft_maps() && as_grouped) ? 1 : 0;
             regroup = full && !adj_recompute && grp.since + 1 >= cic_every;
             a.cnt = regroup ? cic_cnt : nullptr;   // the full push builds the histogram
         }

@@ -679,9 +679,28 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     const size_t plane = a.plane;
     const int tiles_x = My / TX;
     const int j0 = (blockIdx.x % tiles_x) * TX, k0 = (blockIdx.x / tiles_x) * TY;
-    for (int i = threadIdx.x; i < ND * H * W; i += 32 * TY) (&Tt[0][0][0])[i] = zero;
+    const int c0 = j0 + My * (k0 + wr);   // this warp's 32 cells: c0 .. c0+31
+    const int mycell = c0 + lane;
     QS_TRACE_ENTRY();
-    pdl_wait();
+    // The offsets and then the first particles are two dependent loads: they
+    // go first, and the fields' loads and the block's barrier overlap them.
+    // In the march nothing since the kernel before last writes them, so they
+    // need not wait for the kernel in front either.
+    if (!a.early) pdl_wait();
+    const int lo = cell_offset(a, mycell);
+    const int hi = (size_t)(mycell + 1) < plane ? cell_offset(a, mycell + 1) : (int)a.n;
+    for (int i = threadIdx.x; i < ND * H * W; i += 32 * TY) (&Tt[0][0][0])[i] = zero;
+    const int pbeg = __shfl_sync(0xffffffffu, lo, 0);
+    const int pend = __shfl_sync(0xffffffffu, hi, 31);
+    // the particle of the next pass is loaded while this one is pushed
+    int nx_cell = 0;
+    T nx_y = zero, nx_z = zero, nx_px = zero, nx_py = zero, nx_pz = zero, nx_w = zero;
+    if (pbeg + lane < pend) {
+        const int q = pbeg + lane;
+        nx_cell = a.cell[q]; nx_y = a.y[q]; nx_z = a.z[q];
+        nx_px = a.px[q]; nx_py = a.py[q]; nx_pz = a.pz[q]; nx_w = a.w[q];
+    }
+    if (a.early) pdl_wait();
     QS_TRACE_WAITED();
     const bool one_set = a.P == a.C;     // an averaged set: (x + x) / 2 = x
     for (int i = threadIdx.x; i < H * W; i += 32 * TY) {
@@ -717,12 +736,6 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                     a.favg[(2 * q + 1) * plane + m] = Fs[q][r][cc].y;
                 }
             }
-    const int c0 = j0 + My * (k0 + wr);   // this warp's 32 cells: c0 .. c0+31
-    const int mycell = c0 + lane;
-    const int lo = cell_offset(a, mycell);
-    const int hi = (size_t)(mycell + 1) < plane ? cell_offset(a, mycell + 1) : (int)a.n;
-    const int pbeg = __shfl_sync(0xffffffffu, lo, 0);
-    const int pend = __shfl_sync(0xffffffffu, hi, 31);
     const bool count = a.full && a.cnt;
     int stay = 0;                        // particles that end the full push in mycell
     const T dj[4] = {a.djx0, a.djy0, a.djz0, a.drho0};   // the species' factor of each current
@@ -742,14 +755,6 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
             for (int r = 0; r < 4; r++) atomicAdd(a.dep + d * plane + nd[r], x * wc[r]);
         }
     };
-    // the particle of the next pass is loaded while this one is pushed
-    int nx_cell = 0;
-    T nx_y = zero, nx_z = zero, nx_px = zero, nx_py = zero, nx_pz = zero, nx_w = zero;
-    if (pbeg + lane < pend) {
-        const int q = pbeg + lane;
-        nx_cell = a.cell[q]; nx_y = a.y[q]; nx_z = a.z[q];
-        nx_px = a.px[q]; nx_py = a.py[q]; nx_pz = a.pz[q]; nx_w = a.w[q];
-    }
     for (int wbase = pbeg; wbase < pend; wbase += WIN) {
         const int wend = min(pend, wbase + WIN);
         // phase 1: lane = particle

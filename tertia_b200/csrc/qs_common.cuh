@@ -73,6 +73,8 @@ struct PushArgs {
     const int* loff;
     const int* bpref;
     int* cnt;
+    int early;            // 1: the particles and offsets were complete before the kernel in front
+                          // of this one in the launch chain started (they are read before its wait)
     int skip_dens;        // 1: leave out the density deposit (plane 3), unused by the caller
     T* favg;              // grouped CIC without the density deposit: when set, the fields
                           // the push gathers, (P + C) / 2, are written here (6 planes),
