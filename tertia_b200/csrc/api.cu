@@ -1461,6 +1461,7 @@ struct Engine : EngineBase {
         // the fields and the plasma this push reads: with the averaged fields
         // in C the previous layer's last z-pass (side 0) is not among them
         const bool from_avg = !full && half_avg;
+        const bool after_regroup = side_pending[1];
         half_avg = false;
         if (from_avg) join_side(1);
         else join_sides();
@@ -1512,8 +1513,10 @@ struct Engine : EngineBase {
             a.loff = cic_loff;
             a.bpref = cic_bpref;
             // in the march a z-pass (every thread of which waits for the
-            // kernel before it) stands between two pushes
-            a.early = (g_pdl && in_march && !adj_recompute && fft_maps() && as_grouped) ? 1 : 0;
+            // kernel before it) stands between two pushes; a regrouping on
+            // the side stream may end only just before this push
+            a.early = (g_pdl && in_march && !adj_recompute && fft_maps() && as_grouped &&
+                       !after_regroup) ? 1 : 0;
             regroup = full && !adj_recompute && grp.since + 1 >= cic_every;
             a.cnt = regroup ? cic_cnt : nullptr;   // the full push builds the histogram
         }
