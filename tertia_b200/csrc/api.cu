@@ -1615,7 +1615,9 @@ struct Engine : EngineBase {
                 // layer's fields and the predicted ones: with the grouped CIC
                 // push (whose gathered fields the adjoint reads) the map
                 // kernel forms it, so that push needs one z-pass, not two
-                const bool avg = fuse && cic_sort && clear_by_maps();
+                // (without inner iterations the only push is the full one,
+                // which gathers P and C)
+                const bool avg = fuse && cic_sort && clear_by_maps() && nIter > 0;
                 klaunch(KC_SPECTRAL, [&] {
                     return spec_rows_run(a, true, scratch, scratch, nout, fuse ? &an : nullptr,
                                          fuse ? scratch2 : nullptr, avg);
