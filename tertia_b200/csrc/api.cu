@@ -1396,6 +1396,8 @@ struct Engine : EngineBase {
             // predictor and the inverse y-pass of E, B in one kernel, then the z-pass
             SpecArgs<T> a = spec_args(iLayer, iSplit);
             a.zero_src = clear_by_maps() ? Csrc : nullptr;
+            a.skip_dens = (clear_by_maps() && cic_sort) ? 1 : 0;
+            a.lean = in_march ? 1 : 0;
             a.write_b = 0;
             // beside a pending last z-pass of the previous layer (reading
             // scratch) the map writes scratch2
@@ -1598,6 +1600,8 @@ struct Engine : EngineBase {
                 SpecArgs<T> a = spec_args(iLayer, iSplit);
                 a.write_b = 0;
                 a.zero_src = (clear_by_maps() && iter >= 0) ? Csrc : nullptr;
+                a.skip_dens = (clear_by_maps() && cic_sort) ? 1 : 0;
+                a.lean = (in_march && iter >= 0) ? 1 : 0;
                 charge_args(a, iLayer, iSplit, iter);
                 const int nout = want_rho ? 7 : 6;
                 // the layer's last corrector also runs the next layer's
@@ -1609,6 +1613,8 @@ struct Engine : EngineBase {
                     an = spec_args(iLayer - 1, 0);
                     cur ^= 1;
                     an.zero_src = clear_by_maps() ? Psrc : nullptr;   // the next push's deposit
+                    an.skip_dens = a.skip_dens;
+                    an.lean = 1;
                     an.write_b = 0;
                 }
                 // the next layer's first push gathers the average of this

@@ -586,10 +586,26 @@ constexpr int kSpecGroups = 8;
 // kernel, the six field adjoints into its adjoint
 static_assert(kSpecGroups >= 7, "a transform group per plane");
 
+// groups of the warps that transform J's three rows (a warp's groups without
+// a plane run on zeros in their own work space)
+template <int M, class C>
+__host__ __device__ constexpr int spec_jgroups() {
+    constexpr int T = M / spec_vpt<M, C>(), G = T >= 32 ? 1 : 32 / T;
+    return (3 + G - 1) / G * G;
+}
+// work space of the transform groups in C values; behind that of the J groups
+// it also holds three fetched rows
+template <int M, class C>
+__host__ __device__ constexpr int spec_work() {
+    constexpr int LD = M + M / spec_vpt<M, C>();
+    constexpr int need = spec_jgroups<M, C>() * LD + 3 * M;
+    return need > kSpecGroups * LD ? need : kSpecGroups * LD;
+}
+
 template <int M, class C = float2>
 __host__ __device__ constexpr size_t spec_rows_smem() {
     // tables, FFT work of each group, the row's J spectra and E, B, Rho spectra
-    return sizeof(C) * (2 * (size_t)M + (size_t)kSpecGroups * (M + M / spec_vpt<M, C>())) +
+    return sizeof(C) * (2 * (size_t)M + (size_t)spec_work<M, C>()) +
            sizeof(typename Cx<C>::Real) * (3 + 7) * (size_t)(2 * M);
 }
 
@@ -599,13 +615,36 @@ __host__ __device__ constexpr int spec_threads() {
     return kSpecGroups * (M / spec_vpt<M, C>()) > M ? kSpecGroups * (M / spec_vpt<M, C>()) : M;
 }
 
+// 16 bytes from global to shared memory, asynchronously (not through L1)
+__device__ __forceinline__ void cp_async16(void* s, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(s)),
+                 "l"(g)
+                 : "memory");
+}
+
 // PRED_NEXT (with CORRECT): the layer's last corrector, then the next
 // layer's predictor (`an`, whose P bank is the bank the corrector has just
 // written) on the same row, and its inverse y-pass into r.out_next.  The maps
 // are per mode and each thread keeps its mode pairs in both loops, so the
-// predictor reads what the same thread stored; it overwrites the corrector's
-// P bank (no longer needed) only at those modes.  C: float2 (FP32) or
-// double2 (FP64 on FFT transforms).
+// predictor takes the corrector's outputs from the rows in shared memory.  It
+// overwrites the corrector's P bank (no longer needed) only at those modes.
+// C: float2 (FP32) or double2 (FP64 on FFT transforms).
+//
+// What bounds it: the latency of its serial phases (load, y-pass of J, map,
+// inverse y-pass), with four CTAs per SM at ny = 512, more than its traffic.
+// The ten rows the corrector reads (the P bank, the density before, the beam)
+// were complete before the z-pass in front of this kernel started, so they
+// are fetched by cp.async ahead of the wait and land during the y-pass of J,
+// in shared memory that is free until the map: the E, B, Rho rows (the thread
+// that reads a mode pair overwrites it) and the work space of the idle
+// groups.  Of its outputs only those that something reads are stored
+// (SpecArgs::lean).  Against loads in the map, 4 + 3 more planes stored per
+// layer and the predictor's P bank read back from memory: layer of the warm
+// 512 x 512 x 1024 march 96.9 -> 94.4-95.4 us, 1024 x 1024 390 -> 384 us, FP64
+// 512 x 512 183.1 -> 180.8 us.  The predictor in the corrector's own loop, from
+// registers, and all twelve inverse rows behind one barrier was slower (97.7,
+// 403 and 187.7 us: registers).
 template <int M, bool CORRECT, bool PRED_NEXT, class C>
 __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real> a,
                                                    SpecRowArgsT<typename Cx<C>::Real> r,
@@ -624,13 +663,28 @@ __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real
     C* tws = reinterpret_cast<C*>(smem_spec);
     C* posts = tws + M;
     C* W = posts + M;
-    Real* J = reinterpret_cast<Real*>(W + kSpecGroups * LD);   // 3 x N
-    Real* EB = J + 3 * N;                                       // 7 x N
+    Real* J = reinterpret_cast<Real*>(W + spec_work<M, C>());   // 3 x N
+    Real* EB = J + 3 * N;                                        // 7 x N
+    Real* PF = reinterpret_cast<Real*>(W + spec_jgroups<M, C>() * LD);   // 3 fetched rows
+    const int k = blockIdx.x;
+    if constexpr (CORRECT) {
+        constexpr int PP = N * (int)sizeof(Real) / 16;   // pieces of a row
+        static_assert(PP <= NT && NT % PP == 0, "a row's pieces in one go");
+        const Real* src[10] = {a.RhoP, a.JxP, a.JyP, a.JzP, a.EyP, a.EzP, a.Rho,
+                               a.Rb0, a.Jxb0, a.wp0 != Real(0) ? a.Rbp0 : a.Rb0};
+        const int piece = threadIdx.x % PP, lane_row = threadIdx.x / PP;
+#pragma unroll
+        for (int q = 0; q < 10; q++) {
+            Real* dst = q < 7 ? EB + q * N : PF + (q - 7) * N;
+            if (q % (NT / PP) == lane_row)
+                cp_async16(reinterpret_cast<char*>(dst) + 16 * piece,
+                           reinterpret_cast<const char*>(src[q] + (size_t)N * k) + 16 * piece);
+        }
+    }
     for (int i = threadIdx.x; i < M; i += NT) {
         tws[i] = r.tab[i];
         posts[i] = r.tab[2 * M + i];
     }
-    const int k = blockIdx.x;
     const int g = threadIdx.x / T, jt = threadIdx.x % T;
     // the first group of this thread's warp: a warp whose groups all lack a
     // plane skips the transform (its lanes meet no shuffle of another warp)
@@ -654,16 +708,11 @@ __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real
                                 gg == 1 ? QS_RODFT11 : QS_REDFT11, Real(1), valid, jt, Wg, tws,
                                 posts, pre);
         }
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
     }
-    auto to_eb = [&](int j, const Modes2<Real>& o) {
-        *reinterpret_cast<C*>(EB + 0 * N + j) = Cx<C>::make(o.ex[0], o.ex[1]);
-        *reinterpret_cast<C*>(EB + 1 * N + j) = Cx<C>::make(o.ey[0], o.ey[1]);
-        *reinterpret_cast<C*>(EB + 2 * N + j) = Cx<C>::make(o.ez[0], o.ez[1]);
-        *reinterpret_cast<C*>(EB + 3 * N + j) = Cx<C>::make(o.bx[0], o.bx[1]);
-        *reinterpret_cast<C*>(EB + 4 * N + j) = Cx<C>::make(o.by[0], o.by[1]);
-        *reinterpret_cast<C*>(EB + 5 * N + j) = Cx<C>::make(o.bz[0], o.bz[1]);
-        *reinterpret_cast<C*>(EB + 6 * N + j) = Cx<C>::make(o.rho[0], o.rho[1]);
+    auto row2 = [](const Real* rows, int q, int j) {
+        return *reinterpret_cast<const C*>(rows + q * N + j);
     };
     // the maps on the row's modes, two per thread
     double qr = 0.0, qj = 0.0;   // FP64 charge sums (charge.cuh)
@@ -672,13 +721,23 @@ __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real
         const size_t n = (size_t)j + (size_t)N * k;
         Modes2<Real> o;
         if constexpr (CORRECT) {
-            const C jx2 = *reinterpret_cast<const C*>(J + j);
-            const C jy2 = *reinterpret_cast<const C*>(J + N + j);
-            const C jz2 = *reinterpret_cast<const C*>(J + 2 * N + j);
-            st2(const_cast<Real*>(a.Jx), n, jx2.x, jx2.y);   // the bank keeps the deposit spectra
-            st2(const_cast<Real*>(a.Jy), n, jy2.x, jy2.y);
-            st2(const_cast<Real*>(a.Jz), n, jz2.x, jz2.y);
-            o = corrector_modes2(a, j, k, n, jx2, jy2, jz2);
+            const C jx2 = row2(J, 0, j), jy2 = row2(J, 1, j), jz2 = row2(J, 2, j);
+            PBank<Real> p;
+            p.rho = row2(EB, 0, j);
+            p.jx = row2(EB, 1, j);
+            p.jy = row2(EB, 2, j);
+            p.jz = row2(EB, 3, j);
+            p.ey = row2(EB, 4, j);
+            p.ez = row2(EB, 5, j);
+            const C rold = row2(EB, 6, j);
+            const BeamPair<Real> b =
+                beam_mix(a, n, row2(PF, 0, j), row2(PF, 1, j), row2(PF, 2, j));
+            o = corrector_map(a, j, k, p, rold, b, jx2, jy2, jz2);
+            if (!a.lean) {   // the bank keeps the deposit spectra
+                st2(const_cast<Real*>(a.Jx), n, jx2.x, jx2.y);
+                st2(const_cast<Real*>(a.Jy), n, jy2.x, jy2.y);
+                st2(const_cast<Real*>(a.Jz), n, jz2.x, jz2.y);
+            }
             if (a.qsum) {
                 const double c0 = a.qcy[j], c1 = a.qcy[j + 1];
                 qr += (double)o.rho[0] * c0 + (double)o.rho[1] * c1;
@@ -687,8 +746,20 @@ __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real
         } else {
             o = predictor_modes2(a, j, k, n);
         }
-        store_modes2(a, n, o);
-        to_eb(j, o);
+        if (a.lean) {
+            st2(a.Rho, n, o.rho[0], o.rho[1]);
+            zero_src2(a, n);
+        } else {
+            store_modes2(a, n, o);
+        }
+        {
+            const Real v[7][2] = {{o.ex[0], o.ex[1]}, {o.ey[0], o.ey[1]}, {o.ez[0], o.ez[1]},
+                                  {o.bx[0], o.bx[1]}, {o.by[0], o.by[1]}, {o.bz[0], o.bz[1]},
+                                  {o.rho[0], o.rho[1]}};
+#pragma unroll
+            for (int f = 0; f < 7; f++)
+                *reinterpret_cast<C*>(EB + f * N + j) = Cx<C>::make(v[f][0], v[f][1]);
+        }
     }
     if (CORRECT && a.qsum) {
         const double cz = a.qcz[k];
@@ -696,62 +767,65 @@ __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real
     }
     __syncthreads();
     if constexpr (!PRED_NEXT) pdl_trigger();
-    // inverse y-transform of Ex Ey Ez Bx By Bz Rho (y kinds C S C S C S C)
-    if (threadIdx.x < NTF && wg0 < r.nout) {
-        const bool valid = g < r.nout;
-        const int gg = valid ? g : 0;
-        const C* src = reinterpret_cast<const C*>(EB + gg * N);
-        C* dst = reinterpret_cast<C*>(r.out + gg * plane + (size_t)k * N);
-        row_dtt_group<M, C, V>([src](int i) { return src[i]; },
-                            [dst](int q, C v) { dst[q] = v; },
-                            (gg & 1) ? QS_RODFT11 : QS_REDFT11, Real(1), valid, jt, Wg, tws, posts,
-                            pre);
-    }
-    if constexpr (PRED_NEXT) {
-        __syncthreads();   // EB is free again
-        for (int pj = threadIdx.x; pj < M; pj += NT) {
-            const int j = 2 * pj;
-            const size_t n = (size_t)j + (size_t)N * k;
-            const Modes2<Real> o = predictor_modes2(an, j, k, n);
-            store_modes2(an, n, o);
-            if (r.avg_next) {
-                // the fields the next layer's first push gathers: this
-                // layer's (still in EB) and the predicted ones, averaged
-                const Real h = Real(0.5);
-                C* eb = reinterpret_cast<C*>(EB + j);
-                const Real v[6][2] = {{o.ex[0], o.ex[1]}, {o.ey[0], o.ey[1]}, {o.ez[0], o.ez[1]},
-                                      {o.bx[0], o.bx[1]}, {o.by[0], o.by[1]}, {o.bz[0], o.bz[1]}};
-#pragma unroll
-                for (int f = 0; f < 6; f++) {
-                    const C e = eb[f * (N / 2)];
-                    eb[f * (N / 2)] = Cx<C>::make(h * (e.x + v[f][0]), h * (e.y + v[f][1]));
-                }
-            } else {
-                to_eb(j, o);
-            }
-        }
-        __syncthreads();
-        pdl_trigger();
-        if (threadIdx.x < NTF && wg0 < 6) {
-            const bool valid = g < 6;
+    // inverse y-transform of Ex Ey Ez Bx By Bz Rho (y kinds C S C S C S C),
+    // and of the next layer's fields
+    auto inverse = [&](const Real* rows, Real* out, int nout) {
+        if (threadIdx.x < NTF && wg0 < nout) {
+            const bool valid = g < nout;
             const int gg = valid ? g : 0;
-            const C* src = reinterpret_cast<const C*>(EB + gg * N);
-            C* dst = reinterpret_cast<C*>(r.out_next + gg * plane + (size_t)k * N);
+            const C* src = reinterpret_cast<const C*>(rows + gg * N);
+            C* dst = reinterpret_cast<C*>(out + gg * plane + (size_t)k * N);
             row_dtt_group<M, C, V>([src](int i) { return src[i]; },
                                 [dst](int q, C v) { dst[q] = v; },
                                 (gg & 1) ? QS_RODFT11 : QS_REDFT11, Real(1), valid, jt, Wg, tws,
                                 posts, pre);
         }
+    };
+    inverse(EB, r.out, PRED_NEXT ? 6 : r.nout);
+    if constexpr (PRED_NEXT) {
+        __syncthreads();
+        for (int pj = threadIdx.x; pj < M; pj += NT) {
+            const int j = 2 * pj;
+            const size_t n = (size_t)j + (size_t)N * k;
+            // its P bank is what this thread's corrector left in the rows
+            PBank<Real> p;
+            p.rho = row2(EB, 6, j);
+            p.ex = row2(EB, 0, j);
+            p.ey = row2(EB, 1, j);
+            p.ez = row2(EB, 2, j);
+            p.jx = row2(J, 0, j);
+            p.jy = row2(J, 1, j);
+            p.jz = row2(J, 2, j);
+            const Modes2<Real> e = predictor_map(an, j, k, p, beam_pair(an, n));
+            st2(an.Rho, n, e.rho[0], e.rho[1]);   // (an.lean)
+            zero_src2(an, n);
+            const Real v[6][2] = {{e.ex[0], e.ex[1]}, {e.ey[0], e.ey[1]}, {e.ez[0], e.ez[1]},
+                                  {e.bx[0], e.bx[1]}, {e.by[0], e.by[1]}, {e.bz[0], e.bz[1]}};
+            // the next layer's first push gathers this layer's fields and the
+            // predicted ones, averaged (avg_next)
+            const Real h = r.avg_next ? Real(0.5) : Real(1);
+#pragma unroll
+            for (int f = 0; f < 6; f++) {
+                const C c = r.avg_next ? row2(EB, f, j) : Cx<C>::make(Real(0), Real(0));
+                *reinterpret_cast<C*>(EB + f * N + j) =
+                    Cx<C>::make(h * (c.x + v[f][0]), h * (c.y + v[f][1]));
+            }
+        }
+        __syncthreads();
+        pdl_trigger();
+        inverse(EB, r.out_next, 6);
     }
     QS_TRACE_END(PRED_NEXT ? trace::K_MAP_CORR_PRED
                            : (CORRECT ? trace::K_MAP_CORR : trace::K_MAP_PRED));
 }
 
-// On the 1024-wide FP32 grid (M = 512): 512 threads at most 64 registers, two
-// CTAs per SM (their shared memory, 84 KB each, fits twice).
+// Two CTAs per SM where the shared memory of two fits: on the 1024-wide FP32
+// grid (M = 512: 512 threads at most 64 registers; 84 KB each, 108 KB with the
+// next predictor) and on the 512-wide FP64 grid (256 threads at most 128
+// registers; 86 KB, 110 KB).
 template <int M, bool CORRECT, bool PRED_NEXT, class C = float2>
 __global__ void __launch_bounds__(spec_threads<M, C>(),
-                                  (M == 512 && sizeof(C) == sizeof(float2)) ? 2 : 1)
+                                  (M == 512 || (M == 256 && sizeof(C) == sizeof(double2))) ? 2 : 1)
     spectral_rows_kernel(SpecArgs<typename Cx<C>::Real> a, SpecRowArgsT<typename Cx<C>::Real> r,
                          SpecArgs<typename Cx<C>::Real> an) {
     spectral_rows_body<M, CORRECT, PRED_NEXT, C>(a, r, an);

@@ -34,6 +34,13 @@ struct SpecArgs {
     // optional: 4 planes (the C-layer deposit) cleared by the kernel for the
     // push that follows it (ClearCurrentsSplit without a separate memset)
     T* zero_src;
+    int skip_dens;       // 1: the push leaves out the density, whose plane stays clear
+    // 1 (map kernels between the halves of the transforms): of the spectral
+    // outputs only Rho is stored.  The inverse transform takes the fields from
+    // the kernel's own rows, and the next corrector of the layer reads Rho
+    // alone; the layer's last corrector (lean 0) stores the bank the next
+    // layer reads.
+    int lean;
     // optional (correctors): FP64 charge sums (charge.cuh); each block writes
     // its partial sums of rho c_ky c_kz and Jx c_ky c_kz to qsum[2 * block]
     double* qsum;

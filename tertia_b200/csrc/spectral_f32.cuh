@@ -39,10 +39,11 @@ __device__ __forceinline__ void st2(R* p, size_t n, R a, R b) {
 template <class R>
 struct BeamPair { R rb[2], rbp[2], jxb[2]; };
 
+// r, jx, p: the pairs of Rb0, Jxb0 and (used with a nonzero weight) Rbp0
 template <class R>
-__device__ __forceinline__ BeamPair<R> beam_pair(const SpecArgs<R>& a, size_t n) {
+__device__ __forceinline__ BeamPair<R> beam_mix(const SpecArgs<R>& a, size_t n, pair_t<R> r,
+                                                pair_t<R> jx, pair_t<R> p) {
     BeamPair<R> b;
-    pair_t<R> r = ld2(a.Rb0, n), jx = ld2(a.Jxb0, n);
     b.rb[0] = a.wb0 * r.x; b.rb[1] = a.wb0 * r.y;
     b.jxb[0] = a.wb0 * jx.x; b.jxb[1] = a.wb0 * jx.y;
     if (a.wb1 != R(0)) {
@@ -53,8 +54,7 @@ __device__ __forceinline__ BeamPair<R> beam_pair(const SpecArgs<R>& a, size_t n)
     }
     b.rbp[0] = b.rbp[1] = R(0);
     if (a.wp0 != R(0)) {
-        r = ld2(a.Rbp0, n);
-        b.rbp[0] = a.wp0 * r.x; b.rbp[1] = a.wp0 * r.y;
+        b.rbp[0] = a.wp0 * p.x; b.rbp[1] = a.wp0 * p.y;
     }
     if (a.wp1 != R(0)) {
         r = ld2(a.Rbp1, n);
@@ -62,14 +62,22 @@ __device__ __forceinline__ BeamPair<R> beam_pair(const SpecArgs<R>& a, size_t n)
     }
     return b;
 }
+template <class R>
+__device__ __forceinline__ BeamPair<R> beam_pair(const SpecArgs<R>& a, size_t n) {
+    pair_t<R> p;
+    p.x = p.y = R(0);
+    if (a.wp0 != R(0)) p = ld2(a.Rbp0, n);
+    return beam_mix(a, n, ld2(a.Rb0, n), ld2(a.Jxb0, n), p);
+}
 
-// clear two modes of the 4 deposit planes the next push adds to
+// clear two modes of the deposit planes the next push adds to
 template <class R>
 __device__ __forceinline__ void zero_src2(const SpecArgs<R>& a, size_t n) {
     if (a.zero_src) {
         const size_t N = (size_t)a.ny * a.nz;
 #pragma unroll
-        for (int q = 0; q < 4; q++) st2(a.zero_src + q * N, n, R(0), R(0));
+        for (int q = 0; q < 3; q++) st2(a.zero_src + q * N, n, R(0), R(0));
+        if (!a.skip_dens) st2(a.zero_src + 3 * N, n, R(0), R(0));
     }
 }
 
@@ -79,10 +87,17 @@ struct Modes2 {
     R rho[2], ex[2], ey[2], ez[2], bx[2], by[2], bz[2];
 };
 
-// Guess (:843-872) on modes (j, k), (j+1, k); n = j + ny k
+// the P bank's values on two modes
 template <class R>
-__device__ __forceinline__ Modes2<R> predictor_modes2(const SpecArgs<R>& a, int j, int k,
-                                                      size_t n) {
+struct PBank {
+    pair_t<R> rho, ex, ey, ez, jx, jy, jz;
+};
+
+// Guess (:843-872) on modes (j, k), (j+1, k) of the P bank's values p and the
+// beam terms b
+template <class R>
+__device__ __forceinline__ Modes2<R> predictor_map(const SpecArgs<R>& a, int j, int k,
+                                                   const PBank<R>& p, const BeamPair<R>& b) {
     const R d = *a.dens_p, hx = a.hx;
     const R dh2 = d * hx * hx;
     const R inv_den = R(1) / (R(4) + dh2);
@@ -91,13 +106,9 @@ __device__ __forceinline__ Modes2<R> predictor_modes2(const SpecArgs<R>& a, int 
     const R c_ex = R(4) * hx * inv_den;      // 4 Ex hx (k^2 + d) / denominator
     const R c_rho = R(2) * d * hx * inv_den; // 2 (2 rp + rb + rbp) d hx / ((k^2+d) den)
     const R akz = a.piZ * ((R)k + R(0.5));
-    const pair_t<R> rp2 = ld2(a.RhoP, n), jxp2 = ld2(a.JxP, n), jyp2 = ld2(a.JyP, n),
-                    jzp2 = ld2(a.JzP, n), exp2 = ld2(a.ExP, n), eyp2 = ld2(a.EyP, n),
-                    ezp2 = ld2(a.EzP, n);
-    const BeamPair<R> b = beam_pair(a, n);
-    const R rp_[2] = {rp2.x, rp2.y}, jxp_[2] = {jxp2.x, jxp2.y}, jyp_[2] = {jyp2.x, jyp2.y},
-            jzp_[2] = {jzp2.x, jzp2.y}, exp_[2] = {exp2.x, exp2.y},
-            eyp_[2] = {eyp2.x, eyp2.y}, ezp_[2] = {ezp2.x, ezp2.y};
+    const R rp_[2] = {p.rho.x, p.rho.y}, jxp_[2] = {p.jx.x, p.jx.y}, jyp_[2] = {p.jy.x, p.jy.y},
+            jzp_[2] = {p.jz.x, p.jz.y}, exp_[2] = {p.ex.x, p.ex.y}, eyp_[2] = {p.ey.x, p.ey.y},
+            ezp_[2] = {p.ez.x, p.ez.y};
     Modes2<R> o;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -120,23 +131,29 @@ __device__ __forceinline__ Modes2<R> predictor_modes2(const SpecArgs<R>& a, int 
     }
     return o;
 }
-
-// Iterate (:1419-1466) on modes (j, k), (j+1, k) with the C-deposit spectra
-// jx2, jy2, jz2 of the two modes
+// the same with the P bank and the beam spectra read from memory; n = j + ny k
 template <class R>
-__device__ __forceinline__ Modes2<R> corrector_modes2(const SpecArgs<R>& a, int j, int k,
-                                                      size_t n, pair_t<R> jx2, pair_t<R> jy2,
-                                                      pair_t<R> jz2) {
+__device__ __forceinline__ Modes2<R> predictor_modes2(const SpecArgs<R>& a, int j, int k,
+                                                      size_t n) {
+    const PBank<R> p = {ld2(a.RhoP, n), ld2(a.ExP, n), ld2(a.EyP, n), ld2(a.EzP, n),
+                        ld2(a.JxP, n), ld2(a.JyP, n), ld2(a.JzP, n)};
+    return predictor_map(a, j, k, p, beam_pair(a, n));
+}
+
+// Iterate (:1419-1466) on modes (j, k), (j+1, k) of the P bank's values p
+// (its Ex is not used), the density before this iteration, the beam terms and
+// the C-deposit spectra jx2, jy2, jz2
+template <class R>
+__device__ __forceinline__ Modes2<R> corrector_map(const SpecArgs<R>& a, int j, int k,
+                                                   const PBank<R>& p, pair_t<R> rold2,
+                                                   const BeamPair<R>& b, pair_t<R> jx2,
+                                                   pair_t<R> jy2, pair_t<R> jz2) {
     const R d = *a.dens_p, hx = a.hx;
     const R akz = a.piZ * ((R)k + R(0.5));
-    const pair_t<R> rp2 = ld2(a.RhoP, n), jxp2 = ld2(a.JxP, n), jyp2 = ld2(a.JyP, n),
-                    jzp2 = ld2(a.JzP, n), eyp2 = ld2(a.EyP, n), ezp2 = ld2(a.EzP, n),
-                    rold2 = ld2(a.Rho, n);
-    const BeamPair<R> b = beam_pair(a, n);
-    const R rp_[2] = {rp2.x, rp2.y}, jx_[2] = {jx2.x, jx2.y}, jy_[2] = {jy2.x, jy2.y},
-            jz_[2] = {jz2.x, jz2.y}, jxp_[2] = {jxp2.x, jxp2.y}, jyp_[2] = {jyp2.x, jyp2.y},
-            jzp_[2] = {jzp2.x, jzp2.y}, eyp_[2] = {eyp2.x, eyp2.y},
-            ezp_[2] = {ezp2.x, ezp2.y}, rold_[2] = {rold2.x, rold2.y};
+    const R rp_[2] = {p.rho.x, p.rho.y}, jx_[2] = {jx2.x, jx2.y}, jy_[2] = {jy2.x, jy2.y},
+            jz_[2] = {jz2.x, jz2.y}, jxp_[2] = {p.jx.x, p.jx.y}, jyp_[2] = {p.jy.x, p.jy.y},
+            jzp_[2] = {p.jz.x, p.jz.y}, eyp_[2] = {p.ey.x, p.ey.y}, ezp_[2] = {p.ez.x, p.ez.y},
+            rold_[2] = {rold2.x, rold2.y};
     Modes2<R> o;
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -155,6 +172,19 @@ __device__ __forceinline__ Modes2<R> corrector_modes2(const SpecArgs<R>& a, int 
         o.bz[q] = (aky * (jx + b.jxb[q]) - d * o.ey[q]) * inv_ak2;
     }
     return o;
+}
+template <class R>
+__device__ __forceinline__ Modes2<R> corrector_modes2(const SpecArgs<R>& a, int j, int k,
+                                                      size_t n, pair_t<R> jx2, pair_t<R> jy2,
+                                                      pair_t<R> jz2) {
+    PBank<R> p;
+    p.rho = ld2(a.RhoP, n);
+    p.ey = ld2(a.EyP, n);
+    p.ez = ld2(a.EzP, n);
+    p.jx = ld2(a.JxP, n);
+    p.jy = ld2(a.JyP, n);
+    p.jz = ld2(a.JzP, n);
+    return corrector_map(a, j, k, p, ld2(a.Rho, n), beam_pair(a, n), jx2, jy2, jz2);
 }
 
 // Rho, Ex, Ey, Ez (and B when kept) into the spectral bank, and the two modes
