@@ -131,7 +131,7 @@ struct DttFft {
     int ny = 0, nz = 0;
     float2* tab_y = nullptr;   // twiddle tables of each size
     float2* tab_z = nullptr;
-    bool spec_rows = false;    // run_spectral_rows available (ny in [128, 1024])
+    bool spec_rows = false;    // run_spectral_rows available (ny in [64, 1024])
     static DttFft* create(int ny, int nz);   // nullptr when a size is not handled
     int run_pass(int pass, const DttJob<float>& job, float* scratch, cudaStream_t st) const;
     // the z-pass alone: nf planes in -> out, y-spectral or real alike; with
@@ -165,7 +165,7 @@ struct DttFft64 {
     int ny = 0, nz = 0;
     double2* tab_y = nullptr;
     double2* tab_z = nullptr;
-    bool spec_rows = false;    // run_spectral_rows available (ny in [128, 512])
+    bool spec_rows = false;    // run_spectral_rows available (ny in [64, 512])
     static DttFft64* create(int ny, int nz);   // nullptr when a size is not handled
     int run_pass(int pass, const DttJob<double>& job, double* scratch, cudaStream_t st) const;
     // as DttFft's, in FP64
