@@ -369,6 +369,28 @@ struct ColArgsT {
 };
 using ColArgs = ColArgsT<float>;
 
+// 16 bytes from global to shared memory, asynchronously (not through L1)
+__device__ __forceinline__ void cp_async16(void* s, const void* g) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(s)),
+                 "l"(g)
+                 : "memory");
+}
+
+// Whether the column transform brings its tile to shared memory by cp.async
+// (else every thread loads its own values into registers).  Both are bound by
+// latency, about 10 to 20 warps per SM of one load, two or three exchanges
+// and one store.  Staging takes half the registers (62 against 158 at M = 512,
+// where the direct form leaves one CTA on an SM) but adds a trip through
+// shared memory and a barrier.  Layers of a march: 1024 x 1024 382 us direct,
+// 349 us staged; 256 x 256 41.8 and 40.7 us; 512 x 512 95.3 us direct, 96.4 us
+// (8 values per thread) and 98.7 us (16) staged, FP64 180.5 and 183.7 us;
+// the adjoint's accumulating passes at 256 x 256 86.2 and 87.2 us.
+template <int M, bool ACC, class C>
+__host__ __device__ constexpr bool cols_staged() {
+    return M >= 512 || (M == 128 && !ACC && sizeof(C) == sizeof(float2));
+}
+
 // Transform along the strided axis: a CTA takes TJ adjacent columns of one
 // plane (TJ floats = whole 32-byte sectors per row); column c's sequence
 // lives at W[e * TJ + c], its T threads are TJ lanes apart.
@@ -473,21 +495,153 @@ __global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()))
     QS_TRACE_END(trace::K_ZPASS);
 }
 
+// The same with the tile brought to shared memory first (cols_staged).
+template <int M, int TJ, bool ACC, class C>
+__global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()))
+    fft_cols_staged_kernel(ColArgsT<typename Cx<C>::Real> a) {
+    using Real = typename Cx<C>::Real;
+    constexpr int V = vpt_c<M, C>();
+    constexpr int T = M / V;
+    constexpr int NT = TJ * T;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    C* tws = reinterpret_cast<C*>(smem_raw);
+    C* posts = tws + M;
+    C* W = tws + 2 * M;
+    for (int i = threadIdx.x; i < M; i += NT) {
+        tws[i] = a.tab[i];
+        posts[i] = a.tab[2 * M + i];
+    }
+    const int c = threadIdx.x % TJ, jt = threadIdx.x / TJ;
+    const int f = blockIdx.y;
+    const int col = blockIdx.x * TJ + c;
+    const size_t ld = (size_t)a.ncols;
+    auto at = [c](int e) { return e * TJ + c; };
+    const C* pre = a.tab + M;
+    Real lo[V], hi[V];
+    C w[V];
+#pragma unroll
+    for (int b = 0; b < V; b++) w[b] = __ldg(pre + jt + bitrev<V>(b) * T);
+    QS_TRACE_ENTRY();
+    pdl_wait();
+    QS_TRACE_WAITED();
+    const Real* inf = a.in[0];
+    Real* outf = a.out[0];
+    Real* accf = a.acc[0];
+    Real* clrf = a.clr[0];
+    int kind = a.kind[0];
+#pragma unroll
+    for (int q = 1; q < kMaxXfFields; q++)
+        if (q == f) {
+            inf = a.in[q]; outf = a.out[q]; accf = a.acc[q]; clrf = a.clr[q]; kind = a.kind[q];
+        }
+    constexpr int PC = TJ * (int)sizeof(Real) / 16;   // 16-byte pieces of a row
+    Real* IN = reinterpret_cast<Real*>(W);            // gone before W's first store
+    // one pad row per 4 rows: the rows 2 i that neighbouring threads read
+    // start on distinct banks
+    auto row = [](int r) { return (r + (r >> 2)) * TJ; };
+    const Real* src = inf + (size_t)blockIdx.x * TJ;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < 2 * M * PC; i += NT) {
+        const int r = i / PC, p = i % PC;
+        cp_async16(reinterpret_cast<unsigned char*>(IN + row(r)) + 16 * p,
+                   reinterpret_cast<const unsigned char*>(src + (size_t)r * ld) + 16 * p);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < V; b++) {
+        const int i = jt + bitrev<V>(b) * T;
+        lo[b] = IN[row(2 * i) + c];
+        hi[b] = IN[row(2 * M - 1 - 2 * i) + c];
+    }
+    if (ACC && (accf || clrf)) {   // the same for the whole CTA
+#pragma unroll
+        for (int b = 0; b < V; b++) {
+            const int i = jt + bitrev<V>(b) * T;
+            const size_t olo = (size_t)(2 * i) * ld + col;
+            const size_t ohi = (size_t)(2 * M - 1 - 2 * i) * ld + col;
+            if (accf) {
+                accf[olo] += lo[b];
+                accf[ohi] += hi[b];
+            }
+            if (clrf) {
+                clrf[olo] = Real(0);
+                clrf[ohi] = Real(0);
+            }
+        }
+    }
+    C v[V];
+#pragma unroll
+    for (int b = 0; b < V; b++) {
+        const C z = kind == QS_REDFT11 ? Cx<C>::make(lo[b], hi[b]) : Cx<C>::make(hi[b], lo[b]);
+        v[b] = cmul(z, w[b]);
+    }
+    __syncthreads();   // the staged tile is free
+    dft<V>(v);
+    C fin[V];
+    if constexpr (T == 1) {
+#pragma unroll
+        for (int r = 0; r < V; r++) fin[r] = v[r];
+    } else {
+#pragma unroll
+        for (int r = 0; r < V; r++) W[at(jt * V + r)] = v[r];
+        __syncthreads();
+        Passes<M, V, V, false>::run(W, at, jt, tws, fin);
+    }
+    pdl_trigger();
+    Real im[V];
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        const int q = jt + T * m;
+        fin[m] = cmul(fin[m], posts[q]);
+        im[m] = fin[m].y;
+    }
+    __syncthreads();
+    Real* ims = reinterpret_cast<Real*>(W);
+#pragma unroll
+    for (int m = 0; m < V; m++) ims[(jt + T * m) * TJ + c] = im[m];
+    __syncthreads();
+    const Real c2 = Real(2) * a.scale;
+    const Real sgn = kind == QS_REDFT11 ? -c2 : c2;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        const int q = jt + T * m;
+        outf[(size_t)(2 * q) * ld + col] = c2 * fin[m].x;
+        outf[(size_t)(2 * q + 1) * ld + col] = sgn * ims[(M - 1 - q) * TJ + c];
+    }
+    QS_TRACE_END(trace::K_ZPASS);
+}
+
 template <int M, class C = float2>
 __host__ __device__ constexpr int cols_tj() {
     return (M / vpt_c<M, C>()) >= 16 ? 8 : (M / vpt_c<M, C>()) >= 4 ? 16 : 32;
 }
 
-template <int M, class C = float2>
+template <int M, bool ACC, class C = float2>
 size_t cols_smem() {
-    return sizeof(C) * (size_t)M * (2 + cols_tj<M, C>());
+    // the tables, and the work space or the padded input tile in its place
+    return sizeof(C) * (size_t)M * 2 + sizeof(typename Cx<C>::Real) * (size_t)cols_tj<M, C>() *
+                                           (2 * M + (cols_staged<M, ACC, C>() ? M / 2 : 0));
+}
+
+// the column kernel of a launch (ACC: with planes to add to or to clear)
+template <int M, bool ACC, class C>
+constexpr auto cols_fn() {
+    if constexpr (cols_staged<M, ACC, C>()) return fft_cols_staged_kernel<M, cols_tj<M, C>(), ACC, C>;
+    else return fft_cols_kernel<M, cols_tj<M, C>(), C>;
 }
 
 template <int M, class C = float2>
 cudaError_t set_cols_smem() {
-    return cudaFuncSetAttribute(fft_cols_kernel<M, cols_tj<M, C>(), C>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)cols_smem<M, C>());
+    const cudaError_t e = cudaFuncSetAttribute(cols_fn<M, false, C>(),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)cols_smem<M, false, C>());
+    if (e != cudaSuccess) return e;
+    if constexpr (sizeof(C) != sizeof(float2)) return e;   // the adjoint's passes are FP32
+    else
+        return cudaFuncSetAttribute(cols_fn<M, true, C>(),
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)cols_smem<M, true, C>());
 }
 
 template <int M, class C = float2>
@@ -501,8 +655,11 @@ cudaError_t launch_rows(const RowArgsT<typename Cx<C>::Real>& a, cudaStream_t st
 template <int M, class C = float2>
 cudaError_t launch_cols(const ColArgsT<typename Cx<C>::Real>& a, int nf, cudaStream_t st) {
     constexpr int TJ = cols_tj<M, C>();
-    return launch_pdl(fft_cols_kernel<M, TJ, C>, dim3((unsigned)(a.ncols / TJ), (unsigned)nf),
-                      dim3(TJ * (M / vpt_c<M, C>())), cols_smem<M, C>(), st, a);
+    const dim3 grid((unsigned)(a.ncols / TJ), (unsigned)nf), block(TJ * (M / vpt_c<M, C>()));
+    if constexpr (sizeof(C) == sizeof(float2))
+        if (a.acc[0] || a.clr[0])   // the adjoint's passes
+            return launch_pdl(cols_fn<M, true, C>(), grid, block, cols_smem<M, true, C>(), st, a);
+    return launch_pdl(cols_fn<M, false, C>(), grid, block, cols_smem<M, false, C>(), st, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -613,14 +770,6 @@ __host__ __device__ constexpr size_t spec_rows_smem() {
 template <int M, class C = float2>
 __host__ __device__ constexpr int spec_threads() {
     return kSpecGroups * (M / spec_vpt<M, C>()) > M ? kSpecGroups * (M / spec_vpt<M, C>()) : M;
-}
-
-// 16 bytes from global to shared memory, asynchronously (not through L1)
-__device__ __forceinline__ void cp_async16(void* s, const void* g) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                     (unsigned)__cvta_generic_to_shared(s)),
-                 "l"(g)
-                 : "memory");
 }
 
 // PRED_NEXT (with CORRECT): the layer's last corrector, then the next
