@@ -20,6 +20,8 @@
 // reciprocals and FMA contraction allowed: it is instruction bound, not
 // memory bound, and this halves its instruction count.
 #pragma once
+#include <type_traits>
+
 #include "qs_common.cuh"
 #include "qs_internal.h"
 #include "pdl.cuh"
@@ -502,8 +504,8 @@ __global__ void __launch_bounds__(128) push_cell_kernel(PushArgs<float> a) {
 // CIC push over particles grouped by cell (the counting sort in sort.cu
 // regroups them every few full pushes), FP32, or FP64 with FMA contraction
 // for the FP64 path on FFT transforms.  A block owns a tile of 32 x TY cells
-// and stages the fields (P and C averaged) of the tile's cells plus one row
-// and column in shared memory for the gather.  A warp owns one row of 32
+// and stages the fields (P and C averaged) of the tile's cells and the cells
+// around them in shared memory for the gather.  A warp owns one row of 32
 // cells for the whole launch and lane l owns cell c0 + l.  The row's
 // particles are processed in windows of WIN slots:
 //  - phase 1, particle-parallel (lane = particle, the next one prefetched):
@@ -521,8 +523,9 @@ __global__ void __launch_bounds__(128) push_cell_kernel(PushArgs<float> a) {
 // cell's corner sums (the right-hand corners through a shuffle to the next
 // lane), the warps combine their rows in the block tile in two ordered phases,
 // and the tile is flushed, times the species' charge factors, with one global
-// atomic per touched cell and current.  Particles gathered outside the tile
-// (moved since the regrouping) read the fields from global memory.  ND = 3
+// atomic per touched cell and current.  The staged fields reach one cell around
+// the tile, for particles that moved there since the regrouping; the few
+// beyond read the fields from global memory.  ND = 3
 // leaves out the density deposit, which the march does not read.  The full
 // push stores the particles in place with their new cell.  Same physics
 // as push_kernel<T, CIC, precise, fast> (movepart_layer_CIC.cpp:165-193,
@@ -535,7 +538,10 @@ __global__ void __launch_bounds__(128) push_cell_kernel(PushArgs<float> a) {
 // (15.1 M instructions, 64 registers): 103.8 -> 98.3 us per layer of the warm
 // 512 x 512 x 1024 march, 407 -> 398 us at 1024 x 1024, 190.7 -> 186.3 us in
 // FP64.  72 registers, 7 blocks per SM; capped at 64 registers the spills cost
-// more than the eighth block gives (105.0 us).
+// more than the eighth block gives (105.0 us).  The cells around the tile, and
+// 32-bit offsets: 95.3 -> 93.2 us, 256 x 256 adjoint 86.7 -> 85.6 us, 1024 x 1024
+// 349 -> 346 us; the head of the box, where few particles have moved, would be
+// 81.5 without those cells and is 82.2.
 template <class T>
 __device__ __forceinline__ int cell_offset(const PushArgs<T>& a, int c) {
     return a.loff[c] + a.bpref[c >> 10];
@@ -579,6 +585,21 @@ __device__ __forceinline__ void cic_substep(T dy, T dz, T ps, T& ytmp, T& ztmp, 
     wc[1] = ry * (one - rz);
     wc[2] = (one - ry) * rz;
     wc[3] = ry * rz;
+}
+
+// Element i of an array.  In FP32 by a 32-bit byte offset from its base: one
+// address operand for all arrays of a particle or all planes of a node,
+// 95.3 -> 93.2 us per layer of the warm 512 x 512 march (the launch checks that
+// the arrays are below 4 GB).  In FP64, whose registers are full, the plain
+// form (180.7 us against 183.9).
+template <class T, class U>
+__device__ __forceinline__ U* at32(U* base, std::conditional_t<sizeof(T) == 4, unsigned, size_t> i) {
+    if constexpr (sizeof(T) == 4) {
+        using B = std::conditional_t<std::is_const_v<U>, const char, char>;
+        return reinterpret_cast<U*>(reinterpret_cast<B*>(base) + i * 4u);
+    } else {
+        return base + i;
+    }
 }
 
 // (j, k) of a cell, and an index wrapped into its period: bit operations when
@@ -668,15 +689,18 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     using FP = FPair<T>;
     using P2T = typename FP::type;
     constexpr int TX = 32, W = TX + 1, H = TY + 1;
+    constexpr int GW = TX + 3, GH = TY + 3;   // nodes of the tile's cells and their neighbours
     static_assert(WIN % 32 == 0, "whole warps per window");
     const T one = T(1), zero = T(0), half = T(0.5);
-    __shared__ P2T Fs[3][H][W];          // field pairs of the tile cells + one row/column (P, C averaged)
+    __shared__ P2T Fs[3][GH][GW];        // field pairs (P, C averaged) of the tile's cells and one
+                                         // cell around them
     __shared__ T Tt[ND][H][W];           // block deposit tile [current][row][col]
     __shared__ DepositStage<T, ND, WIN> S[TY];   // staged deposits of each warp's window
     __shared__ int Kl[TY][WIN + WIN / 32];       // counting push: the final cells
     const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
     const int My = a.My, Mz = a.Mz;
-    const size_t plane = a.plane;
+    using Off = std::conditional_t<sizeof(T) == 4, unsigned, size_t>;
+    const Off plane = (Off)a.plane;
     const int tiles_x = My / TX;
     const int j0 = (blockIdx.x % tiles_x) * TX, k0 = (blockIdx.x / tiles_x) * TY;
     const int c0 = j0 + My * (k0 + wr);   // this warp's 32 cells: c0 .. c0+31
@@ -688,7 +712,7 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     // need not wait for the kernel in front either.
     if (!a.early) pdl_wait();
     const int lo = cell_offset(a, mycell);
-    const int hi = (size_t)(mycell + 1) < plane ? cell_offset(a, mycell + 1) : (int)a.n;
+    const int hi = (Off)(mycell + 1) < plane ? cell_offset(a, mycell + 1) : (int)a.n;
     for (int i = threadIdx.x; i < ND * H * W; i += 32 * TY) (&Tt[0][0][0])[i] = zero;
     const int pbeg = __shfl_sync(0xffffffffu, lo, 0);
     const int pend = __shfl_sync(0xffffffffu, hi, 31);
@@ -696,30 +720,36 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     int nx_cell = 0;
     T nx_y = zero, nx_z = zero, nx_px = zero, nx_py = zero, nx_pz = zero, nx_w = zero;
     if (pbeg + lane < pend) {
-        const int q = pbeg + lane;
-        nx_cell = a.cell[q]; nx_y = a.y[q]; nx_z = a.z[q];
-        nx_px = a.px[q]; nx_py = a.py[q]; nx_pz = a.pz[q]; nx_w = a.w[q];
+        const Off q = pbeg + lane;
+        nx_cell = *at32<T>(a.cell, q); nx_y = *at32<T>(a.y, q); nx_z = *at32<T>(a.z, q);
+        nx_px = *at32<T>(a.px, q); nx_py = *at32<T>(a.py, q); nx_pz = *at32<T>(a.pz, q);
+        nx_w = *at32<T>(a.w, q);
     }
     if (a.early) pdl_wait();
     QS_TRACE_WAITED();
     const bool one_set = a.P == a.C;     // an averaged set: (x + x) / 2 = x
-    for (int i = threadIdx.x; i < H * W; i += 32 * TY) {
-        const int r = i / W, cc = i - r * W;
-        const size_t m = (size_t)wrap_p<P2>(j0 + cc, My) + (size_t)My * wrap_p<P2>(k0 + r, Mz);
-        if (one_set) {
+    {
+        int r = threadIdx.x / GW, cc = threadIdx.x - r * GW;
+        for (int i = threadIdx.x; i < GH * GW; i += 32 * TY) {
+            const Off m = (Off)wrap_p<P2>(j0 + cc - 1, My) + (Off)My * wrap_p<P2>(k0 + r - 1, Mz);
+            if (one_set) {
 #pragma unroll
-            for (int q = 0; q < 3; q++)
-                Fs[q][r][cc] =
-                    FP::make(ld(a.C + 2 * q * plane + m), ld(a.C + (2 * q + 1) * plane + m));
-        } else {
+                for (int q = 0; q < 3; q++)
+                    Fs[q][r][cc] = FP::make(ld(at32<T>(a.C + 2 * q * plane, m)),
+                                            ld(at32<T>(a.C + (2 * q + 1) * plane, m)));
+            } else {
 #pragma unroll
-            for (int q = 0; q < 3; q++) {
-                const P2T pp =
-                    FP::make(ld(a.P + 2 * q * plane + m), ld(a.P + (2 * q + 1) * plane + m));
-                const P2T cp =
-                    FP::make(ld(a.C + 2 * q * plane + m), ld(a.C + (2 * q + 1) * plane + m));
-                Fs[q][r][cc] = FP::mul(half, FP::add(pp, cp));
+                for (int q = 0; q < 3; q++) {
+                    const P2T pp = FP::make(ld(at32<T>(a.P + 2 * q * plane, m)),
+                                            ld(at32<T>(a.P + (2 * q + 1) * plane, m)));
+                    const P2T cp = FP::make(ld(at32<T>(a.C + 2 * q * plane, m)),
+                                            ld(at32<T>(a.C + (2 * q + 1) * plane, m)));
+                    Fs[q][r][cc] = FP::mul(half, FP::add(pp, cp));
+                }
             }
+            cc += (32 * TY) % GW;      // the node 32 * TY further
+            r += (32 * TY) / GW;
+            if (cc >= GW) { cc -= GW; r += 1; }
         }
     }
     __syncthreads();
@@ -729,11 +759,11 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
         if (a.favg)
             for (int i = threadIdx.x; i < TY * TX; i += 32 * TY) {
                 const int r = i / TX, cc = i - r * TX;
-                const size_t m = (size_t)(j0 + cc) + (size_t)My * (k0 + r);
+                const Off m = (Off)(j0 + cc) + (Off)My * (k0 + r);
 #pragma unroll
                 for (int q = 0; q < 3; q++) {
-                    a.favg[2 * q * plane + m] = Fs[q][r][cc].x;
-                    a.favg[(2 * q + 1) * plane + m] = Fs[q][r][cc].y;
+                    a.favg[2 * q * plane + m] = Fs[q][r + 1][cc + 1].x;
+                    a.favg[(2 * q + 1) * plane + m] = Fs[q][r + 1][cc + 1].y;
                 }
             }
     const bool count = a.full && a.cnt;
@@ -746,13 +776,13 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     // the 4 corners of cell (jc, kc) get q[d] * dj[d] * weight by global atomics
     auto scatter = [&](int jc, int kc, const T (&q)[ND], const T (&wc)[4]) {
         const int jc1 = wrap_p<P2>(jc + 1, My), kc1 = wrap_p<P2>(kc + 1, Mz);
-        const size_t nd[4] = {(size_t)jc + (size_t)My * kc, (size_t)jc1 + (size_t)My * kc,
-                              (size_t)jc + (size_t)My * kc1, (size_t)jc1 + (size_t)My * kc1};
+        const Off nd[4] = {(Off)(jc + My * kc), (Off)(jc1 + My * kc), (Off)(jc + My * kc1),
+                           (Off)(jc1 + My * kc1)};
 #pragma unroll
         for (int d = 0; d < ND; d++) {
             const T x = q[d] * dj[d];
 #pragma unroll
-            for (int r = 0; r < 4; r++) atomicAdd(a.dep + d * plane + nd[r], x * wc[r]);
+            for (int r = 0; r < 4; r++) atomicAdd(at32<T>(a.dep + d * plane, nd[r]), x * wc[r]);
         }
     };
     for (int wbase = pbeg; wbase < pend; wbase += WIN) {
@@ -764,9 +794,10 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
             const T yp = nx_y, zp = nx_z, w = nx_w;
             T px = nx_px, py = nx_py, pz = nx_pz;
             if (p + 32 < pend) {
-                const int q = p + 32;
-                nx_cell = a.cell[q]; nx_y = a.y[q]; nx_z = a.z[q];
-                nx_px = a.px[q]; nx_py = a.py[q]; nx_pz = a.pz[q]; nx_w = a.w[q];
+                const Off q = p + 32;
+                nx_cell = *at32<T>(a.cell, q); nx_y = *at32<T>(a.y, q); nx_z = *at32<T>(a.z, q);
+                nx_px = *at32<T>(a.px, q); nx_py = *at32<T>(a.py, q); nx_pz = *at32<T>(a.pz, q);
+                nx_w = *at32<T>(a.w, q);
             }
             int key = -1, last = cell;
             T qv[ND], ay = zero, az = zero;
@@ -781,8 +812,14 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                     const T wg[4] = {(one - yp) * (one - zp), yp * (one - zp), (one - yp) * zp,
                                      yp * zp};
                     T g[6];
-                    const int tj = j - j0, tk = k - k0;
-                    if ((unsigned)tj < TX && (unsigned)tk < TY) {
+                    // the particle's node in the tile (moved since the regrouping,
+                    // it may sit in a cell around the tile's own)
+                    int tj = j - j0 + 1, tk = k - k0 + 1;
+                    if constexpr (P2) {   // across the periodic edge too
+                        tj &= My - 1;
+                        tk &= Mz - 1;
+                    }
+                    if ((unsigned)tj < TX + 2 && (unsigned)tk < TY + 2) {
 #pragma unroll
                         for (int q = 0; q < 3; q++) {
                             P2T gq = FP::mul(wg[0], Fs[q][tk][tj]);
@@ -794,17 +831,15 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                         }
                     } else {
                         const int j1 = wrap_p<P2>(j + 1, My), k1 = wrap_p<P2>(k + 1, Mz);
-                        const size_t nn[4] = {(size_t)j + (size_t)My * k,
-                                              (size_t)j1 + (size_t)My * k,
-                                              (size_t)j + (size_t)My * k1,
-                                              (size_t)j1 + (size_t)My * k1};
+                        const Off nn[4] = {(Off)(j + My * k), (Off)(j1 + My * k),
+                                           (Off)(j + My * k1), (Off)(j1 + My * k1)};
 #pragma unroll
                         for (int f = 0; f < 6; f++) {
                             T s = zero;
 #pragma unroll
                             for (int r = 0; r < 4; r++)
-                                s += wg[r] * half * (ld(a.P + f * plane + nn[r]) +
-                                                     ld(a.C + f * plane + nn[r]));
+                                s += wg[r] * half * (ld(at32<T>(a.P + f * plane, nn[r])) +
+                                                     ld(at32<T>(a.C + f * plane, nn[r])));
                             g[f] = s;
                         }
                     }
@@ -870,8 +905,10 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                     }
                     last = jb + My * kb;
                     if (a.full) {
-                        a.y[p] = ytmp; a.z[p] = ztmp; a.px[p] = px; a.py[p] = py; a.pz[p] = pz;
-                        a.cell_out[p] = last;
+                        const Off q = p;
+                        *at32<T>(a.y, q) = ytmp; *at32<T>(a.z, q) = ztmp; *at32<T>(a.px, q) = px;
+                        *at32<T>(a.py, q) = py; *at32<T>(a.pz, q) = pz;
+                        *at32<T>(a.cell_out, q) = last;
                     }
                 }
             }
@@ -952,14 +989,17 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
         if (lane == 31) Tt[d][wr + 1][TX] += edge1[d];
     }
     __syncthreads();
+    int fr = threadIdx.x / W, fc = threadIdx.x - fr * W;
     for (int i = threadIdx.x; i < H * W; i += 32 * TY) {
-        const int r = i / W, cc = i - r * W;
-        const size_t m = (size_t)wrap_p<P2>(j0 + cc, My) + (size_t)My * wrap_p<P2>(k0 + r, Mz);
+        const Off m = (Off)wrap_p<P2>(j0 + fc, My) + (Off)My * wrap_p<P2>(k0 + fr, Mz);
 #pragma unroll
         for (int d = 0; d < ND; d++) {
-            const T x = Tt[d][r][cc];
-            if (x != zero) atomicAdd(a.dep + d * plane + m, dj[d] * x);
+            const T x = Tt[d][fr][fc];
+            if (x != zero) atomicAdd(at32<T>(a.dep + d * plane, m), dj[d] * x);
         }
+        fc += (32 * TY) % W;
+        fr += (32 * TY) / W;
+        if (fc >= W) { fc -= W; fr += 1; }
     }
     QS_TRACE_END(a.full ? trace::K_PUSH_FULL : trace::K_PUSH_HALF);
 }
@@ -969,6 +1009,8 @@ template <class T>
 int launch_push_rows(const PushArgs<T>& a, cudaStream_t st) {
     constexpr int TY = 4, WIN = 128;
     if (!a.loff || a.dep_cell) return 0;   // grouped by cell with offsets (the engine checks the shape)
+    // 32-bit byte offsets into the particle arrays and the planes
+    if ((uint64_t)a.n * sizeof(T) >= (1ull << 32) || (uint64_t)a.plane * sizeof(T) >= (1ull << 32)) return 0;
     const dim3 grid((a.My / 32) * (a.Mz / TY));
     const dim3 block(32 * TY);
     if (a.skip_dens) {

@@ -78,3 +78,36 @@ def test_row_push_edges(oracle_lib, prec, ny, nz, hy):
         assert rel_l2(dep, np.asarray(r["dep"], float)[:3]) < td
         if sums is not None:   # each particle keeps its own weight through the regrouping
             np.testing.assert_array_equal(sums, p["w"])
+
+
+# the second push starts from the first one's positions, TOL's tx off at most:
+# so are its weights, and a node's sum is off by about as much relative to it
+TOL2 = {"fp32": 1e-4, "fp64fft": 1e-11}
+
+
+@pytest.mark.parametrize("prec,ny,nz,hy", [("fp32", 32, 32, 0.2), ("fp32", 64, 8, 0.01),
+                                           ("fp32", 96, 24, 0.2), ("fp32", 96, 40, 0.01),
+                                           ("fp64fft", 64, 32, 0.2), ("fp64fft", 32, 64, 0.01)])
+def test_row_push_after_a_move(oracle_lib, prec, ny, nz, hy):
+    """Particles that left the cell they are grouped by: into the cells around
+    their tile, across the periodic edges and further."""
+    from tertia_b200.mesh import Mesh
+    cfg = cfg_for(prec, n=32, layers=4, shape=QS_SHAPE_CIC)
+    cfg.ny, cfg.nz, cfg.hy, cfg.hz = ny, nz, hy, hy
+    p, P, C = crowd(cfg, 3 * ny + nz)
+    dt = np.float32 if prec == "fp32" else np.float64
+    with Mesh(cfg) as m:
+        m.load_front_plasma(p)
+        for c in range(6):
+            m.set_layer(QS_LAYER_P, c, P[c])
+            m.set_layer(QS_LAYER_C, c, C[c])
+        m.move_particles_layer(0, 0, 1)
+        m.move_particles_layer(0, 0, 0)
+        dep = np.stack([m.get_layer(QS_LAYER_C, f) for f in (QS_F_JX, QS_F_JY, QS_F_JZ)])
+    r = {k: (np.asarray(v, dt) if k != "cell" else v) for k, v in p.items()}
+    w = r["w"]
+    for full in (True, False):
+        r = oracle_lib.push_layer(cfg, r["cell"], r["y"], r["z"], r["px"], r["py"], r["pz"], w,
+                                  P.astype(dt), C.astype(dt), full=full, precise=True, dtype=dt)
+    assert np.mean(np.asarray(r["cell"]) != p["cell"]) > 0.05
+    assert rel_l2(dep, np.asarray(r["dep"], float)[:3]) < TOL2[prec]
