@@ -310,10 +310,16 @@ struct Engine : EngineBase {
         bool grouped = true, off_valid = false, counted = false, flip = false;
         int since = 0;   // full pushes since the last regrouping
     } grp;
-    // regroup after every cic_every-th full push (particles drift about 1% of
-    // a cell per layer, so the push's global-memory fallback for the few that
-    // left their row stays cheap in between); QS_CIC_REGROUP overrides
-    int cic_every = getenv("QS_CIC_REGROUP") ? std::max(1, atoi(getenv("QS_CIC_REGROUP"))) : 2;
+    // Regroup after every cic_every-th full push: a regrouping costs about 8 us
+    // of a 512 x 512 layer, and particles that left their cell since the last
+    // one cost the push some atomics.  With the wake and thermal drift of the
+    // usual decks (about 1% of a cell per layer) every 4th is best at 512 and
+    // 1024 (us per layer every 2 / 4 / 8: warm 512 x 512 x 1024 93.2 / 91.3 /
+    // 91.1, 1024 x 1024 346 / 332 / 328, FP64 180.7 / 177.3 / 176.5; 256 x 256
+    // 40.5 / 40.6 / 40.9).  A thermal move of 5% of a cell per layer breaks even
+    // (100.1 / 99.5 at every 2 / 4), 10% does not (105.6 / 109.5), so from 6%
+    // on it is every 2nd (set in init).  QS_CIC_REGROUP overrides.
+    int cic_every = 4;
     // programmatic dependent launch inside the march (QS_PDL=0 turns it off)
     bool use_pdl = !(getenv("QS_PDL") && getenv("QS_PDL")[0] == '0');
     bool uniform_layout = false;   // particle p in cell p / ppc (lattice seeding)
@@ -345,6 +351,7 @@ struct Engine : EngineBase {
     // a segment, the position adjoint, and the reorder between checkpoints
     bool cic_adj = false;
     bool adj_recompute = false;   // recomputing a segment: keep the particle order
+    int* ck_off = nullptr;        // the cell offsets of each checkpoint's particle order
     int32_t *ck_cell = nullptr, *ck_id = nullptr, *seg_cell = nullptr, *adj_inv = nullptr;
     T* lam_pos = nullptr;
     T* adj_tmp = nullptr;
@@ -405,7 +412,7 @@ struct Engine : EngineBase {
                         stage, stage_d, pcell, py, pz, ppx, ppy, ppz, pw, bi, bj, bk, bx, by, bz,
                         bpx, bpy, bpz, bw, d_err, dens_dev, front_src, front_beam, ck, seg, lam, lam_pm, lam_sb,
                         d_dloss, d_gradw, acell, pid, apid, ay, az, apx, apy, apz, aw, cic_cnt,
-                        cic_loff, cic_bsum, cic_bpref, cic_ticket, ck_cell, ck_id, seg_cell,
+                        cic_loff, cic_bsum, cic_bpref, cic_ticket, ck_off, ck_cell, ck_id, seg_cell,
                         adj_inv, lam_pos, adj_tmp, d_pack, d_pack_i, q_cy, q_cz, q_part,
                         qb_part, q_sums, study_f, study_p, scratch2, fstore};
         for (void* p : ptrs)
@@ -459,6 +466,12 @@ struct Engine : EngineBase {
         cic_sort = cfg.shape == QS_SHAPE_CIC &&
                    (sizeof(T) == 4 || cfg.precision == QS_PREC_FP64_FFT) && My % 32 == 0 &&
                    Mz % 4 == 0;
+        {
+            const double sp = std::max(std::fabs(cfg.pspread_y), std::fabs(cfg.pspread_z));
+            const double drift = sp * cfg.hx / S / std::min(cfg.hy, cfg.hz);
+            cic_every = drift < 0.06 ? 4 : 2;
+            if (const char* e = getenv("QS_CIC_REGROUP")) cic_every = std::max(1, atoi(e));
+        }
         if (cic_sort) {
             const int nb_scan = scan_blocks_count((int)plane);
             if ((s = alloc(&cic_cnt, plane, "cell counts"))) return s;
@@ -2191,6 +2204,7 @@ struct Engine : EngineBase {
     // carries along) and the P-bank spectra (Rho, Ex, Ey, Ez, Jx, Jy, Jz);
     // the P-layer fields are layer L-m*K of the field store.
     size_t ck_stride() const { return 6 * (size_t)adj_np + 7 * plane; }
+    size_t off_stride() const { return plane + (size_t)scan_blocks_count((int)plane) + 1; }
     size_t seg_stride() const { return 5 * (size_t)adj_np + (size_t)(nIter + 1) * 6 * plane; }
     T* particle_arrays(int c) { T* a[5] = {py, pz, ppx, ppy, ppz}; return a[c]; }
 
@@ -2212,9 +2226,18 @@ struct Engine : EngineBase {
         if (cic_adj) {   // CIC: the cells move, and the plasma is regrouped (ids)
             CK(cudaMemcpyAsync(ck_cell + (size_t)m * np, pcell, np * sizeof(int32_t),
                                cudaMemcpyDeviceToDevice, st));
-            if (cic_sort)
+            if (cic_sort) {
                 CK(cudaMemcpyAsync(ck_id + (size_t)m * np, pid, np * sizeof(int32_t),
                                    cudaMemcpyDeviceToDevice, st));
+                // the offsets of this order, whose grouping may be some pushes
+                // old (offsets counted from the current cells would not fit it)
+                if (qs_status s = cic_prepare()) return s;
+                int* off = ck_off + (size_t)m * off_stride();
+                CK(cudaMemcpyAsync(off, cic_loff, plane * sizeof(int), cudaMemcpyDeviceToDevice,
+                                   st));
+                CK(cudaMemcpyAsync(off + plane, cic_bpref, (off_stride() - plane) * sizeof(int),
+                                   cudaMemcpyDeviceToDevice, st));
+            }
         }
         return QS_OK;
     }
@@ -2240,11 +2263,14 @@ struct Engine : EngineBase {
             if (cic_sort) {
                 CK(cudaMemcpyAsync(pid, ck_id + (size_t)m * np, np * sizeof(int32_t),
                                    cudaMemcpyDeviceToDevice, st));
-                // the recomputation keeps this order (no regrouping): fresh
-                // counts and offsets for it
-                CK(cudaMemsetAsync(cic_cnt, 0, plane * sizeof(int), st));
+                // the recomputation keeps this order (no regrouping) and its offsets
+                const int* off = ck_off + (size_t)m * off_stride();
+                CK(cudaMemcpyAsync(cic_loff, off, plane * sizeof(int), cudaMemcpyDeviceToDevice,
+                                   st));
+                CK(cudaMemcpyAsync(cic_bpref, off + plane, (off_stride() - plane) * sizeof(int),
+                                   cudaMemcpyDeviceToDevice, st));
                 grp.grouped = true;
-                grp.off_valid = false;
+                grp.off_valid = true;
                 grp.counted = false;
                 grp.since = 0;
             }
@@ -2261,13 +2287,13 @@ struct Engine : EngineBase {
             return fail(QS_ERR_UNSUPPORTED, "the adjoint needs 6 ny nz and 3 x the particle count "
                                             "below 2^31");
         CK(cudaStreamSynchronize(st));
-        void* old[] = {ck, seg, lam, lam_pm, lam_sb, d_dloss, ck_cell, ck_id, seg_cell,
+        void* old[] = {ck, seg, lam, lam_pm, lam_sb, d_dloss, ck_off, ck_cell, ck_id, seg_cell,
                        lam_pos, adj_inv, adj_tmp, fstore};
         for (void* p : old)
             if (p) cudaFree(p);
         ck = seg = lam = lam_pm = lam_sb = d_dloss = lam_pos = adj_tmp = fstore = nullptr;
         lam_lo = -1;
-        ck_cell = ck_id = seg_cell = adj_inv = nullptr;
+        ck_off = ck_cell = ck_id = seg_cell = adj_inv = nullptr;
         ck_every = 0;
         ck_valid = false;
         if (gexec) {   // the captured march has (or lacks) the checkpoint copies
@@ -2293,6 +2319,8 @@ struct Engine : EngineBase {
             if ((s = alloc(&lam_pos, 2 * (size_t)np, "adjoint positions"))) return s;
             if (cic_sort) {
                 if ((s = alloc(&ck_id, (size_t)ck_count * np, "adjoint checkpoints"))) return s;
+                if ((s = alloc(&ck_off, (size_t)ck_count * off_stride(), "adjoint checkpoints")))
+                    return s;
                 if ((s = alloc(&adj_inv, (size_t)np, "adjoint reorder"))) return s;
                 if ((s = alloc(&adj_tmp, 5 * (size_t)np, "adjoint reorder"))) return s;
             }
