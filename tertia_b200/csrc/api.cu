@@ -36,6 +36,7 @@ namespace qs {
 
 static thread_local std::string g_create_error;
 thread_local bool g_pdl = false;
+thread_local bool g_capturing = false;
 
 // error text of calls made without a handle (read by qs_last_error(NULL))
 void set_unbound_error(const std::string& why) { g_create_error = why; }
@@ -1171,7 +1172,17 @@ struct Engine : EngineBase {
         }
     }
 
+    // the launch chain of a run of FFT passes outside the march (their kernels
+    // wait for the one in front before they touch its planes)
+    struct PdlScope {
+        bool old = g_pdl;
+        explicit PdlScope(bool on) { g_pdl = g_pdl || on; }
+        ~PdlScope() { g_pdl = old; }
+    };
+    bool chain_fft() const { return (fftx || fftx64) && use_pdl && !prof && !fp32_study; }
+
     qs_status beam_spectra() {
+        PdlScope chain(chain_fft());
         klaunch(KC_BEAM_SPECTRA, [&] {
             return launch_beam_check<T>(b3, L + 1, plane, d_err, qb_part, st);
         });
@@ -2166,10 +2177,10 @@ struct Engine : EngineBase {
             graph_front = front_layer;
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            capturing = true;
+            capturing = g_capturing = true;
             capture_count = 0;
             qs_status s = march_device();
-            capturing = false;
+            capturing = g_capturing = false;
             cudaError_t e = cudaStreamEndCapture(st, &g);
             if (s) {
                 if (g) cudaGraphDestroy(g);
@@ -2789,12 +2800,12 @@ struct Engine : EngineBase {
                 adj_exec = nullptr;
                 cudaGraph_t g = nullptr;
                 CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-                capturing = true;
+                capturing = g_capturing = true;
                 capture_count = 0;
                 g_pdl = use_pdl;
                 qs_status s = adjoint_device(lo);
                 g_pdl = false;
-                capturing = false;
+                capturing = g_capturing = false;
                 cudaError_t e = cudaStreamEndCapture(st, &g);
                 if (s) {
                     if (g) cudaGraphDestroy(g);
@@ -2858,6 +2869,7 @@ struct Engine : EngineBase {
             return fail(QS_ERR_INVALID, "qs_transform2d_dev: bad arguments");
         const T* in = (const T*)d_in;
         T* out = (T*)d_out;
+        PdlScope chain(chain_fft());
         for (int b0 = 0; b0 < batch; b0 += kMaxXfFields) {
             int nf = std::min(kMaxXfFields, batch - b0);
             T* outs[kMaxXfFields];

@@ -237,6 +237,7 @@ using RowArgs = RowArgsT<float>;
 
 template <int M, class C = float2>
 __host__ __device__ constexpr int row_threads() {
+    if (sizeof(C) == sizeof(double2) && M >= 256) return 128;
     return (M / vpt_c<M, C>()) > 64 ? (M / vpt_c<M, C>()) : 64;
 }
 

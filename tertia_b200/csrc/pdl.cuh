@@ -16,8 +16,10 @@
 
 namespace qs {
 
-// set by the engine around the launches of a march (per host thread)
+// set by the engine around the launches of a march (per host thread), and
+// while it captures a graph
 extern thread_local bool g_pdl;
+extern thread_local bool g_capturing;
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() {
@@ -39,10 +41,10 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         n++;
     }
-    // the stream's priority, also as a node attribute when the launch is
-    // captured into a graph
+    // the stream's priority as a node attribute when the launch is captured
+    // into a graph (outside a capture the stream itself carries it)
     int prio = 0;
-    if (cudaStreamGetPriority(st, &prio) == cudaSuccess && prio != 0) {
+    if (g_capturing && cudaStreamGetPriority(st, &prio) == cudaSuccess && prio != 0) {
         attr[n].id = cudaLaunchAttributePriority;
         attr[n].val.priority = prio;
         n++;
