@@ -699,13 +699,21 @@ struct Engine : EngineBase {
                                           (double)job.scale, st);
                 });
         } else if (fftx) {
-            if constexpr (sizeof(T) == 4)
+            if constexpr (sizeof(T) == 4) {
+                if (fftx->planes &&
+                    klaunch(KC_GEMM, [&] { return fftx->run_planes(job, st); }))
+                    return;
                 for (int pass = 0; pass < 2; pass++)
                     klaunch(KC_GEMM, [&] { return fftx->run_pass(pass, job, work, st); });
+            }
         } else if (fftx64) {
-            if constexpr (sizeof(T) == 8)
+            if constexpr (sizeof(T) == 8) {
+                if (fftx64->planes &&
+                    klaunch(KC_GEMM, [&] { return fftx64->run_planes(job, st); }))
+                    return;
                 for (int pass = 0; pass < 2; pass++)
                     klaunch(KC_GEMM, [&] { return fftx64->run_pass(pass, job, work, st); });
+            }
         } else {
             for (int pass = 0; pass < 2; pass++)
                 klaunch(KC_GEMM, [&] {

@@ -24,6 +24,8 @@
 #include <cmath>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "qs_common.cuh"
 #include "qs_internal.h"
 #include "pdl.cuh"
@@ -1032,6 +1034,170 @@ cudaError_t launch_spec_rows(const SpecArgs<typename Cx<C>::Real>& a,
     return launch_pdl(spec_rows_fn<M, false, false, C>(), grid, block, sm, st, a, r, a);
 }
 
+// ---------------------------------------------------------------------------
+// The whole 2-D transform of a small plane (sizes 32 to 128) in one launch: a
+// cluster of CL CTAs per plane, 4096 values each.  A CTA takes its share of the
+// rows through the y-pass and puts each result, transposed, into the shared
+// memory of the CTA that owns its column; behind the cluster's barrier every
+// CTA takes its columns through the z-pass into the destination.  Every CTA
+// has read its rows before that barrier, so a plane may be transformed in
+// place.  A batch of such planes is bound by launches and latency, so one
+// launch instead of two, back to back on one stream: 3 planes of 128 x 128 FP32
+// 6.1 -> 4.5 us per call (one CTA per plane: 8.0), 64 x 64 6.1 -> 4.9 us, FP64
+// 64 x 64 6.0 -> 4.2 us; FP64 128 x 128, 6.0 -> 6.4 us, keeps two launches.
+constexpr int kPlaneThreads = 256;
+
+template <class Real>
+struct PlaneArgsT {
+    const Real* in[kMaxXfFields];
+    Real* out[kMaxXfFields];
+    int ky[kMaxXfFields], kz[kMaxXfFields];
+    Real scale;
+    const typename CxOf<Real>::type *tab_y, *tab_z;
+};
+
+template <int MY, int MZ>
+__host__ __device__ constexpr int plane_cluster() {
+    return MY * MZ > 1024 ? MY * MZ / 1024 : 1;
+}
+template <int MY, int MZ, class C>
+__host__ __device__ constexpr int plane_work() {
+    constexpr int wy = kPlaneThreads / (MY / 8) * (MY + MY / 8);
+    constexpr int wz = kPlaneThreads / (MZ / 8) * (MZ + MZ / 8);
+    return wy > wz ? wy : wz;
+}
+template <int MY, int MZ, class C>
+constexpr size_t plane_smem() {
+    return sizeof(C) * (size_t)(2 * MY + 2 * MZ + plane_work<MY, MZ, C>()) +
+           sizeof(typename Cx<C>::Real) * (size_t)(2 * MY / plane_cluster<MY, MZ>()) * (2 * MZ + 1);
+}
+
+template <int MY, int MZ, class C>
+__global__ void __cluster_dims__(plane_cluster<MY, MZ>(), 1, 1) __launch_bounds__(kPlaneThreads)
+    fft_plane_kernel(PlaneArgsT<typename Cx<C>::Real> a) {
+    using Real = typename Cx<C>::Real;
+    constexpr int NY = 2 * MY, NZ = 2 * MZ, LDP = NZ + 1, CL = plane_cluster<MY, MZ>();
+    constexpr int RZ = NZ / CL, RY = NY / CL;   // rows and columns of a CTA
+    extern __shared__ __align__(16) unsigned char smem_plane[];
+    C* twy = reinterpret_cast<C*>(smem_plane);
+    C* posty = twy + MY;
+    C* twz = posty + MY;
+    C* postz = twz + MZ;
+    C* W = postz + MZ;
+    Real* P = reinterpret_cast<Real*>(W + plane_work<MY, MZ, C>());   // [own column][z]
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = CL > 1 ? (int)cluster.block_rank() : 0;
+    if constexpr (CL > 1) cg::this_cluster().barrier_arrive();   // this CTA's memory exists
+    for (int i = threadIdx.x; i < MY; i += kPlaneThreads) {
+        twy[i] = a.tab_y[i];
+        posty[i] = a.tab_y[2 * MY + i];
+    }
+    for (int i = threadIdx.x; i < MZ; i += kPlaneThreads) {
+        twz[i] = a.tab_z[i];
+        postz[i] = a.tab_z[2 * MZ + i];
+    }
+    const int f = blockIdx.x / CL;
+    const Real* in = a.in[0];
+    Real* out = a.out[0];
+    int ky = a.ky[0], kz = a.kz[0];
+#pragma unroll
+    for (int q = 1; q < kMaxXfFields; q++)
+        if (q == f) { in = a.in[q]; out = a.out[q]; ky = a.ky[q]; kz = a.kz[q]; }
+    pdl_wait();
+    __syncthreads();
+    if constexpr (CL > 1) cg::this_cluster().barrier_wait();
+    {
+        constexpr int T = MY / 8, G = kPlaneThreads / T;
+        const int g = threadIdx.x / T, jt = threadIdx.x % T;
+        for (int r0 = 0; r0 < RZ; r0 += G) {
+            const bool valid = r0 + g < RZ;
+            const int k = rank * RZ + (valid ? r0 + g : 0);
+            const C* src = reinterpret_cast<const C*>(in + (size_t)k * NY);
+            row_dtt_group<MY, C, 8>(
+                [src](int i) { return src[i]; },
+                [&](int q, C v) {
+                    const int j = 2 * q;   // RY is even: both values have one owner
+                    Real* D = P;
+                    if constexpr (CL > 1) D = cluster.map_shared_rank(P, j / RY);
+                    D[(j % RY) * LDP + k] = v.x;
+                    D[(j % RY + 1) * LDP + k] = v.y;
+                },
+                ky, Real(1), valid, jt, W + g * (MY + MY / 8), twy, posty, a.tab_y + MY);
+        }
+    }
+    if constexpr (CL > 1) cluster.sync();
+    else __syncthreads();
+    pdl_trigger();
+    {
+        constexpr int T = MZ / 8, G = kPlaneThreads / T;
+        const int g = threadIdx.x / T, jt = threadIdx.x % T;
+        for (int c0 = 0; c0 < RY; c0 += G) {
+            const bool valid = c0 + g < RY;
+            const int c = valid ? c0 + g : 0, j = rank * RY + c;
+            const Real* src = P + c * LDP;
+            row_dtt_group<MZ, C, 8>(
+                [src](int i) { return Cx<C>::make(src[2 * i], src[2 * i + 1]); },
+                [&](int q, C v) {
+                    out[(size_t)(2 * q) * NY + j] = v.x;
+                    out[(size_t)(2 * q + 1) * NY + j] = v.y;
+                },
+                kz, a.scale, valid, jt, W + g * (MZ + MZ / 8), twz, postz, a.tab_z + MZ);
+        }
+    }
+}
+
+// calls f with the kernel of the sizes (both among 32, 64, 128)
+template <class C, class F>
+cudaError_t with_plane_kernel(int ny, int nz, F&& f) {
+#define QS_PLANE(Y, Z)                 \
+    if (ny == 2 * (Y) && nz == 2 * (Z)) \
+        return f(fft_plane_kernel<Y, Z, C>, plane_smem<Y, Z, C>());
+    QS_PLANE(16, 16) QS_PLANE(16, 32) QS_PLANE(16, 64)
+    QS_PLANE(32, 16) QS_PLANE(32, 32) QS_PLANE(32, 64)
+    QS_PLANE(64, 16) QS_PLANE(64, 32) QS_PLANE(64, 64)
+#undef QS_PLANE
+    return cudaErrorInvalidValue;
+}
+inline bool plane_size_ok(int n) { return n == 32 || n == 64 || n == 128; }
+
+template <class C>
+bool set_plane_smem(int ny, int nz) {
+    if (!plane_size_ok(ny) || !plane_size_ok(nz)) return false;
+    if (sizeof(C) == sizeof(double2) && ny * nz > 8192) return false;
+    return with_plane_kernel<C>(ny, nz, [](auto fn, size_t smem) {
+               return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem);
+           }) == cudaSuccess;
+}
+
+// the job in one launch; 0 when a plane's output overlaps another plane's input
+template <class C>
+int launch_planes(const DttJob<typename Cx<C>::Real>& job, int ny, int nz, const C* tab_y,
+                  const C* tab_z, cudaStream_t st) {
+    using Real = typename Cx<C>::Real;
+    const size_t plane = (size_t)ny * nz;
+    PlaneArgsT<Real> a{};
+    for (int f = 0; f < job.nf; f++) {
+        for (int g = 0; g < job.nf; g++) {
+            const bool apart = job.out[f] + plane <= job.in[g] || job.in[g] + plane <= job.out[f];
+            if (!apart && !(f == g && job.out[f] == job.in[f])) return 0;
+        }
+        a.in[f] = job.in[f];
+        a.out[f] = job.out[f];
+        a.ky[f] = job.ky[f];
+        a.kz[f] = job.kz[f];
+    }
+    a.scale = job.scale;
+    a.tab_y = tab_y;
+    a.tab_z = tab_z;
+    const int cl = plane > 4096 ? (int)(plane / 4096) : 1;   // plane_cluster
+    const cudaError_t e = with_plane_kernel<C>(ny, nz, [&](auto fn, size_t smem) {
+        return launch_pdl(fn, dim3((unsigned)(job.nf * cl)), dim3(kPlaneThreads), smem, st, a);
+    });
+    return e == cudaSuccess ? 1 : 0;
+}
+
 // The adjoints of the maps in the same arrangement (the transforms are their
 // own transposes): a CTA takes z-mode row k of the six field adjoints (after
 // their z-pass) through the y-pass, the corrector's (or predictor's) adjoint
@@ -1256,7 +1422,13 @@ DttFft* DttFft::create(int ny, int nz) {
         delete d;
         return nullptr;
     }
+    d->planes = fft::set_plane_smem<float2>(ny, nz);
     return d;
+}
+
+int DttFft::run_planes(const DttJob<float>& job, cudaStream_t st) const {
+    if (!planes || job.nf <= 0 || job.nf > kMaxXfFields) return 0;
+    return fft::launch_planes<float2>(job, ny, nz, tab_y, tab_z, st);
 }
 
 int DttFft::run_cols(int nf, const float* const* in, float* const* out, const int* kind,
@@ -1431,7 +1603,13 @@ DttFft64* DttFft64::create(int ny, int nz) {
         d->spec_rows = e == cudaSuccess;
         cudaGetLastError();
     }
+    d->planes = fft::set_plane_smem<double2>(ny, nz);
     return d;
+}
+
+int DttFft64::run_planes(const DttJob<double>& job, cudaStream_t st) const {
+    if (!planes || job.nf <= 0 || job.nf > kMaxXfFields) return 0;
+    return fft::launch_planes<double2>(job, ny, nz, tab_y, tab_z, st);
 }
 
 int DttFft64::run_cols(int nf, const double* const* in, double* const* out, const int* kind,
