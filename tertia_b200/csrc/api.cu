@@ -257,6 +257,17 @@ struct Engine : EngineBase {
     // next Guess, so its first push gathers from C alone and does not wait for
     // the layer's last z-pass (side stream 0)
     bool next_avg = false, half_avg = false;
+    // Up to 256 x 256 the last z-pass of a layer waits for the next Guess and runs
+    // in one launch with its z-pass (12 planes) instead of on a side stream:
+    // one launch less, no competition with the chain, and no fork and join in
+    // the captured graph, whose instantiation they cost about 50 us a layer.
+    // Per layer 64 x 64 NGP 22.1 -> 21.1 us, 128 x 128 31.0 -> 30.4, 256 x 256
+    // 40.7 -> 38.6; a handle's first march of 256 x 256 x 128 layers 17.3 -> 9.9
+    // ms.  At 512 x 512 the side stream is faster (91.3 against 92.2 us, FP64 177.3
+    // against 180.4) though a first march of 1024 layers would take 122 ms
+    // instead of 184.
+    bool merge_z = false;       // set for one march
+    T* zp_out = nullptr;        // the six planes a waiting z-pass (from scratch) writes
     int fuse_lo = 0;            // lowest layer of the march (or recomputed segment)
     // adjoint sweep: the predictor adjoint of a layer runs on side stream 0
     // beside the next layer's first field z-pass (which then uses scratch2)
@@ -1418,7 +1429,8 @@ struct Engine : EngineBase {
             pred_next = -1;
             half_avg = next_avg;
             next_avg = false;
-            eb_zpass(6, scratch2);
+            if (zp_out) eb_zpass_pair();
+            else eb_zpass(6, scratch2);
             CK(cudaGetLastError());
             return QS_OK;
         }
@@ -1484,6 +1496,27 @@ struct Engine : EngineBase {
         const int kz[7] = {CC, CC, SS, SS, SS, CC, CC};
         for (int f = 0; f < nout; f++) ins[f] = from + (size_t)f * plane;
         klaunch(KC_GEMM, [&] { return cols_run(nout, ins, outs, kz, inv_scale()); });
+    }
+
+    // the waiting z-pass of the previous layer (scratch into zp_out) and this
+    // layer's (scratch2 into the C layer) in one launch
+    void eb_zpass_pair() {
+        const T* ins[12];
+        T* outs[12];
+        int kz[12];
+        const int k6[6] = {CC, CC, SS, SS, SS, CC};
+        for (int f = 0; f < 6; f++) {
+            ins[f] = scratch2 + (size_t)f * plane;
+            outs[f] = Cf + (size_t)f * plane;
+            ins[6 + f] = scratch + (size_t)f * plane;
+            outs[6 + f] = zp_out + (size_t)f * plane;
+            kz[f] = kz[6 + f] = k6[f];
+        }
+        zp_out = nullptr;
+        klaunch(KC_GEMM, [&] {
+            if constexpr (sizeof(T) == 4) return fftx->run_cols_pair(ins, outs, kz, inv_scale(), st);
+            else return fftx64->run_cols_pair(ins, outs, kz, inv_scale(), st);
+        });
     }
 
     // Inside the march (no source store) the deposit planes are cleared by
@@ -1662,7 +1695,9 @@ struct Engine : EngineBase {
                 });
                 pred_next = fuse ? iLayer - 1 : -1;
                 next_avg = avg;
-                if (side_z && iter < 0 && nout == 6) {
+                if (fuse && merge_z) {
+                    zp_out = Cf;   // with the next Guess
+                } else if (side_z && !merge_z && iter < 0 && nout == 6) {
                     // the layer's last z-pass: only the next layer's pushes read it
                     const cudaError_t e = on_side(0, [&] { eb_zpass(nout, scratch); });
                     if (e != cudaSuccess) return cuda_fail(e, "side stream");
@@ -1907,13 +1942,16 @@ struct Engine : EngineBase {
         // side streams: not under per-kernel event timing or the precision study
         const bool side = !prof && !fp32_study;
         side_z = side && (fft_maps() || fftx64) && S == 1 && !src3;
+        merge_z = side_z && fft_maps() && My <= 256 && Mz <= 256;
+        zp_out = nullptr;
         side_sort = side && cic_sort;
         pred_next = -1;
         next_avg = half_avg = false;
         fuse_lo = 0;
         qs_status s = march_device_body();
         join_sides();
-        side_z = side_sort = false;
+        side_z = side_sort = merge_z = false;
+        zp_out = nullptr;
         pred_next = -1;
         next_avg = half_avg = false;
         g_pdl = false;
@@ -2441,6 +2479,8 @@ struct Engine : EngineBase {
         // the forward's side stream for the last z-pass of a layer and its
         // fused next predictor (the plasma is not regrouped here)
         side_z = !prof && !fp32_study && (fft_maps() || fftx64) && S == 1 && !src3;
+        merge_z = side_z && fft_maps() && My <= 256 && Mz <= 256;
+        zp_out = nullptr;
         pred_next = -1;
         next_avg = half_avg = false;
         fuse_lo = lo;
@@ -2470,7 +2510,8 @@ struct Engine : EngineBase {
             if ((s = layer_end(i, 0))) break;
         }
         join_sides();
-        side_z = false;
+        side_z = merge_z = false;
+        zp_out = nullptr;
         pred_next = -1;
         next_avg = half_avg = false;
         fuse_lo = 0;

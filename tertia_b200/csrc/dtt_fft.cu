@@ -359,13 +359,13 @@ __global__ void __launch_bounds__(row_threads<M, C>())
     for (int m = 0; m < V; m++) O[jt + T * m] = Cx<C>::make(c2 * fin[m].x, sgn * mirror[m]);
 }
 
-template <class Real>
+template <class Real, int NF = kMaxXfFields>
 struct ColArgsT {
-    const Real* in[kMaxXfFields];
-    Real* out[kMaxXfFields];
-    Real* acc[kMaxXfFields];    // optional: the input is also added here
-    Real* clr[kMaxXfFields];    // optional: the input planes, zeroed once read
-    int kind[kMaxXfFields];
+    const Real* in[NF];
+    Real* out[NF];
+    Real* acc[NF];              // optional: the input is also added here
+    Real* clr[NF];              // optional: the input planes, zeroed once read
+    int kind[NF];
     int ncols;                // row length of the planes (the y size)
     Real scale;
     const typename CxOf<Real>::type* tab;
@@ -397,9 +397,9 @@ __host__ __device__ constexpr bool cols_staged() {
 // Transform along the strided axis: a CTA takes TJ adjacent columns of one
 // plane (TJ floats = whole 32-byte sectors per row); column c's sequence
 // lives at W[e * TJ + c], its T threads are TJ lanes apart.
-template <int M, int TJ, class C>
+template <int M, int TJ, class C, int NF = kMaxXfFields>
 __global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()))
-    fft_cols_kernel(ColArgsT<typename Cx<C>::Real> a) {
+    fft_cols_kernel(ColArgsT<typename Cx<C>::Real, NF> a) {
     using Real = typename Cx<C>::Real;
     constexpr int V = vpt_c<M, C>();
     constexpr int T = M / V;
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()))
     Real* clrf = a.clr[0];
     int kind = a.kind[0];
 #pragma unroll
-    for (int q = 1; q < kMaxXfFields; q++)
+    for (int q = 1; q < NF; q++)
         if (q == f) {
             inf = a.in[q]; outf = a.out[q]; accf = a.acc[q]; clrf = a.clr[q]; kind = a.kind[q];
         }
@@ -663,6 +663,41 @@ cudaError_t launch_cols(const ColArgsT<typename Cx<C>::Real>& a, int nf, cudaStr
         if (a.acc[0] || a.clr[0])   // the adjoint's passes
             return launch_pdl(cols_fn<M, true, C>(), grid, block, cols_smem<M, true, C>(), st, a);
     return launch_pdl(cols_fn<M, false, C>(), grid, block, cols_smem<M, false, C>(), st, a);
+}
+
+// The z-passes of two layers' E, B in one launch (12 planes), up to nz = 256
+// (the direct form; no planes to add to or clear).
+constexpr int kPairPlanes = 12;
+template <int M, class C>
+cudaError_t launch_cols_pair(const ColArgsT<typename Cx<C>::Real, kPairPlanes>& a,
+                             cudaStream_t st) {
+    constexpr int TJ = cols_tj<M, C>();
+    static_assert(sizeof(C) * (size_t)M * (2 + TJ) <= 48 * 1024, "no opt-in to larger shared memory");
+    return launch_pdl(fft_cols_kernel<M, TJ, C, kPairPlanes>,
+                      dim3((unsigned)(a.ncols / TJ), (unsigned)kPairPlanes),
+                      dim3(TJ * (M / vpt_c<M, C>())), sizeof(C) * (size_t)M * (2 + TJ), st, a);
+}
+template <class C>
+int run_cols_pair(int ny, int nz, const typename Cx<C>::Real* const* in,
+                  typename Cx<C>::Real* const* out, const int* kind,
+                  typename Cx<C>::Real scale, const C* tab, cudaStream_t st) {
+    ColArgsT<typename Cx<C>::Real, kPairPlanes> a{};
+    for (int f = 0; f < kPairPlanes; f++) {
+        a.in[f] = in[f];
+        a.out[f] = out[f];
+        a.kind[f] = kind[f];
+    }
+    a.ncols = ny;
+    a.scale = scale;
+    a.tab = tab;
+    cudaError_t e;
+    switch (nz / 2) {
+        case 128: e = launch_cols_pair<128, C>(a, st); break;
+        case 64: e = launch_cols_pair<64, C>(a, st); break;
+        case 32: e = launch_cols_pair<32, C>(a, st); break;
+        default: e = launch_cols_pair<16, C>(a, st); break;
+    }
+    return e == cudaSuccess ? 1 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1431,6 +1466,11 @@ int DttFft::run_planes(const DttJob<float>& job, cudaStream_t st) const {
     return fft::launch_planes<float2>(job, ny, nz, tab_y, tab_z, st);
 }
 
+int DttFft::run_cols_pair(const float* const* in, float* const* out, const int* kind, float scale,
+                          cudaStream_t st) const {
+    return fft::run_cols_pair<float2>(ny, nz, in, out, kind, scale, tab_z, st);
+}
+
 int DttFft::run_cols(int nf, const float* const* in, float* const* out, const int* kind,
                      float scale, cudaStream_t st, float* const* acc, float* const* clr) const {
     if (nf <= 0 || nf > kMaxXfFields) return 0;
@@ -1610,6 +1650,11 @@ DttFft64* DttFft64::create(int ny, int nz) {
 int DttFft64::run_planes(const DttJob<double>& job, cudaStream_t st) const {
     if (!planes || job.nf <= 0 || job.nf > kMaxXfFields) return 0;
     return fft::launch_planes<double2>(job, ny, nz, tab_y, tab_z, st);
+}
+
+int DttFft64::run_cols_pair(const double* const* in, double* const* out, const int* kind,
+                            double scale, cudaStream_t st) const {
+    return fft::run_cols_pair<double2>(ny, nz, in, out, kind, scale, tab_z, st);
 }
 
 int DttFft64::run_cols(int nf, const double* const* in, double* const* out, const int* kind,

@@ -143,6 +143,9 @@ struct DttFft {
     int run_cols(int nf, const float* const* in, float* const* out, const int* kind, float scale,
                  cudaStream_t st, float* const* acc = nullptr,
                  float* const* clr = nullptr) const;
+    // the z-pass of 12 planes in one launch (nz at most 256)
+    int run_cols_pair(const float* const* in, float* const* out, const int* kind, float scale,
+                      cudaStream_t st) const;
     // one z-mode row per CTA: [forward y-pass of the 3 z-transformed deposit
     // planes at jin, when `correct`] -> corrector (or predictor) of `a` ->
     // inverse y-pass of Ex Ey Ez Bx By Bz (, Rho when nout = 7) into `out`
@@ -176,6 +179,8 @@ struct DttFft64 {
     // as DttFft's, in FP64
     int run_cols(int nf, const double* const* in, double* const* out, const int* kind,
                  double scale, cudaStream_t st) const;
+    int run_cols_pair(const double* const* in, double* const* out, const int* kind, double scale,
+                      cudaStream_t st) const;
     int run_spectral_rows(const SpecArgs<double>& a, bool correct, const double* jin, double* out,
                           int nout, cudaStream_t st, const SpecArgs<double>* next = nullptr,
                           double* out_next = nullptr, bool avg_next = false) const;
