@@ -437,6 +437,7 @@ __device__ __forceinline__ int push_adjoint_cic_one(const PushAdjArgs<T>& a, uin
     }
 
     // ---- backward through the sub-steps: deposits and position chain
+    if (a.early) pdl_wait();
     T lyc = a.full ? a.lamPos[i] : T(0), lzc = a.full ? a.lamPos[un + i] : T(0);
     T ldy = T(0), ldz = T(0), lstep = T(0);
     T ldq[3] = {T(0), T(0), T(0)};
@@ -618,15 +619,20 @@ __device__ __forceinline__ bool warp_run_sums(V (&v)[NV], int key) {
     return key >= 0 && lane == rs;
 }
 
-// FP32: 4 blocks per SM (64 registers and a few spills; the latency of the
-// gathers hidden by more warps, measured faster than 2 or 3 blocks); FP64 as
-// many registers as it takes
+// FP32: 32 warps per SM (64 registers and a few spills; the latency of the
+// gathers hidden by more warps, measured faster than 16 or 24) in blocks of
+// 128 threads (finer than 256 at the end of the last wave: 512 x 512 228.8 ->
+// 225.0 us per adjoint layer); FP64 as many registers as it takes.  In the
+// sweep the particles and the gathered fields are long complete, so the
+// recomputation of the push runs ahead of the wait for the z-pass in front,
+// which brings the current adjoints.
+constexpr int kAdjThreads = 128;
 template <class T>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(kAdjThreads, sizeof(T) == 4 ? 1024 / kAdjThreads : 1)
     push_adjoint_cic_kernel(PushAdjArgs<T> a) {
-    __shared__ T sg[12 * 256];
+    __shared__ T sg[12 * kAdjThreads];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    pdl_wait();
+    if (!a.early) pdl_wait();
     typename FPair<T>::type lf[12];
     int j = 0, k = 0;
     const int cell = i < (uint32_t)a.n ? push_adjoint_cic_one(a, i, lf, j, k, sg) : -1;
@@ -636,6 +642,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
     }
     // the field adjoints of a cell's particles summed in the warp, then one
     // atomic per field and corner
+    pdl_wait();      // (a lane without a particle has not waited yet)
+    pdl_trigger();
     if (warp_run_sums<12>(lf, cell)) {
         const int My = a.My, Mz = a.Mz;
         const uint32_t plane = (uint32_t)a.plane;
@@ -657,7 +665,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 1)
 template <class T>
 int launch_push_adjoint_cic(const PushAdjArgs<T>& a, cudaStream_t st) {
     if (a.n <= 0) return 0;
-    launch_pdl(push_adjoint_cic_kernel<T>, dim3((unsigned)((a.n + 255) / 256)), dim3(256), 0, st,
+    launch_pdl(push_adjoint_cic_kernel<T>,
+               dim3((unsigned)((a.n + kAdjThreads - 1) / kAdjThreads)), dim3(kAdjThreads), 0, st,
                a);
     return 1;
 }
@@ -781,12 +790,14 @@ int launch_avg_planes(const T* P, const T* C, T* out, size_t n, cudaStream_t st)
 // out[idx] += v[layer] for the on-axis loss gradient of one layer
 template <class T>
 __global__ void add_point_kernel(T* plane_ex, size_t idx, const T* v, int layer) {
+    pdl_wait();
+    pdl_trigger();
     if (threadIdx.x == 0 && blockIdx.x == 0) plane_ex[idx] += v[layer];
 }
 
 template <class T>
 int launch_add_point(T* plane_ex, size_t idx, const T* v, int layer, cudaStream_t st) {
-    add_point_kernel<T><<<1, 32, 0, st>>>(plane_ex, idx, v, layer);
+    launch_pdl(add_point_kernel<T>, dim3(1), dim3(32), 0, st, plane_ex, idx, v, layer);
     return 1;
 }
 

@@ -45,19 +45,20 @@ __device__ __forceinline__ void corrector_adjoint_mode(const AdjSpecArgs<T>& a, 
     const T akz = a.piZ * (T(k) + T(0.5));
     const T aky = a.piY * (T(j) + T(0.5));
     const T k2 = aky * aky + akz * akz;
+    const T ik2 = T(1) / k2, idk = T(1) / (d + k2);   // the mode's two reciprocals
     const T lrho = opt(a.lRho, n);
     const T lex = le[0] + opt(a.lEb[0], n);
     T ley = le[1] + opt(a.lEb[1], n);
     T lez = le[2] + opt(a.lEb[2], n);
     const T lbx = lb[0], lby = lb[1], lbz = lb[2];
     // by = (-akz (jx + jxb) + d ez)/k2, bz = (aky (jx + jxb) - d ey)/k2
-    lez += d * lby / k2;
-    ley -= d * lbz / k2;
-    const T ljxs = (-akz * lby + aky * lbz) / k2;          // d(by,bz)/d(jx + jxb)
+    lez += d * lby * ik2;
+    ley -= d * lbz * ik2;
+    const T ljxs = (-akz * lby + aky * lbz) * ik2;          // d(by,bz)/d(jx + jxb)
     T ljx = lrho + ljxs + opt(a.lJb[0], n);
-    T ljy = -hx * T(0.5) * aky * lrho - aky / k2 * lex + akz / k2 * lbx + opt(a.lJb[1], n);
-    T ljz = -hx * T(0.5) * akz * lrho - akz / k2 * lex - aky / k2 * lbx + opt(a.lJb[2], n);
-    const T lsrc = (aky * ley + akz * lez) / (d + k2);     // src = rb + rbp + rp + rho_old
+    T ljy = -hx * T(0.5) * aky * lrho - aky * ik2 * lex + akz * ik2 * lbx + opt(a.lJb[1], n);
+    T ljz = -hx * T(0.5) * akz * lrho - akz * ik2 * lex - aky * ik2 * lbx + opt(a.lJb[2], n);
+    const T lsrc = (aky * ley + akz * lez) * idk;     // src = rb + rbp + rp + rho_old
     lj[0] = ljx;
     lj[1] = ljy;
     lj[2] = ljz;
@@ -84,17 +85,18 @@ __device__ __forceinline__ void predictor_adjoint_mode(const AdjSpecArgs<T>& a, 
     const T akz = a.piZ * (T(k) + T(0.5));
     const T aky = a.piY * (T(j) + T(0.5));
     const T k2 = aky * aky + akz * akz;
-    const T den = T(4) + d * hx * hx;
-    const T prop = (T(4) - d * hx * hx) / den;
+    const T ik2 = T(1) / k2, idk = T(1) / (d + k2);   // the mode's two reciprocals
+    const T iden = T(1) / (T(4) + d * hx * hx);
+    const T prop = (T(4) - d * hx * hx) * iden;
     const T lrho = opt(a.lRho, n);
     T lex = le[0], ley = le[1], lez = le[2];
     const T lbx = lb[0], lby = lb[1], lbz = lb[2];
     // b from the predicted currents and fields
-    const T ljx = (-akz * lby + aky * lbz) / k2;   // also the jxb adjoint
-    const T ljy = akz * lbx / k2;
-    const T ljz = -aky * lbx / k2;
-    lez += d * lby / k2;
-    ley -= d * lbz / k2;
+    const T ljx = (-akz * lby + aky * lbz) * ik2;   // also the jxb adjoint
+    const T ljy = akz * lbx * ik2;
+    const T ljz = -aky * lbx * ik2;
+    lez += d * lby * ik2;
+    ley -= d * lbz * ik2;
     // jx = jxp + hx d (ex + exp)/2 (and y, z)
     const T hd2 = hx * d * T(0.5);
     lex += hd2 * ljx;
@@ -102,16 +104,16 @@ __device__ __forceinline__ void predictor_adjoint_mode(const AdjSpecArgs<T>& a, 
     lez += hd2 * ljz;
     T lexp = hd2 * ljx, leyp = hd2 * ljy, lezp = hd2 * ljz;
     // ey = -eyp + aky src/(d + k2), src = rb + rbp + rp + rho
-    const T lsrc = (aky * ley + akz * lez) / (d + k2);
+    const T lsrc = (aky * ley + akz * lez) * idk;
     leyp -= ley;
     lezp -= lez;
     const T lrho_t = lrho + lsrc;
     // rho = prop rp - (rb + rbp) d hx^2/den + 4 exp hx (k2 + d)/den
     // ex  = prop exp - 2 (2 rp + rb + rbp) d hx / ((k2 + d) den)
-    const T cex = T(2) * d * hx / ((k2 + d) * den);
+    const T cex = T(2) * d * hx * idk * iden;
     const T lrp = lsrc + prop * lrho_t - T(2) * cex * lex;
-    const T lrb = lsrc - d * hx * hx / den * lrho_t - cex * lex;
-    lexp += T(4) * hx * (k2 + d) / den * lrho_t + prop * lex;
+    const T lrb = lsrc - d * hx * hx * iden * lrho_t - cex * lex;
+    lexp += T(4) * hx * (k2 + d) * iden * lrho_t + prop * lex;
     put_lp(a, 0, n, lrp);
     put_lp(a, 1, n, lexp);
     put_lp(a, 2, n, leyp);

@@ -278,14 +278,14 @@ struct Engine : EngineBase {
     // push is the grouped CIC one, for the fstore_n layers nearest the head
     // that fit in free device memory (all of them where they fit): the adjoint
     // recomputes a segment whose layers are all stored by its full pushes
-    // alone, each gathering the stored fields (the march's pushes, bit for
-    // bit), instead of by the whole march.  The adjoint sweeps from the head
+    // alone, each gathering the stored fields (the march's moves), instead
+    // of by the whole march.  The adjoint sweeps from the head
     // down to the loss window, so the head layers are the ones it reads.
     // QS_ADJ_FIELDS=n stores at most n layers (0: no store).
     T* fstore = nullptr;
     int fstore_n = 0;
     long fstore_cap = getenv("QS_ADJ_FIELDS") ? atol(getenv("QS_ADJ_FIELDS")) : -1;
-    const T* push_fields = nullptr;   // the next push gathers these planes alone
+    const T* adj_w = nullptr;         // the weights of the segment the sweep is in
     T* mats = nullptr;          // transform matrices
     DttMats<T> my, mz;
     TcTransformer* tcx = nullptr;
@@ -424,7 +424,7 @@ struct Engine : EngineBase {
                         stage, stage_d, pcell, py, pz, ppx, ppy, ppz, pw, bi, bj, bk, bx, by, bz,
                         bpx, bpy, bpz, bw, d_err, dens_dev, front_src, front_beam, ck, seg, lam, lam_pm, lam_sb,
                         d_dloss, d_gradw, acell, pid, apid, ay, az, apx, apy, apz, aw, cic_cnt,
-                        cic_loff, cic_bsum, cic_bpref, cic_ticket, ck_off, ck_cell, ck_id, seg_cell,
+                        cic_loff, cic_bsum, cic_bpref, cic_ticket, ck_cell, ck_id, seg_cell,
                         adj_inv, lam_pos, adj_tmp, d_pack, d_pack_i, q_cy, q_cz, q_part,
                         qb_part, q_sums, study_f, study_p, scratch2, fstore};
         for (void* p : ptrs)
@@ -1523,6 +1523,26 @@ struct Engine : EngineBase {
     // the spectral kernel that precedes each push instead of by a memset.
     bool clear_by_maps() const { return in_march && !src3; }
 
+    // the sizes and the physics of a push
+    PushArgs<T> push_args() {
+        PushArgs<T> a{};
+        a.n = np;
+        a.My = My; a.Mz = Mz;
+        a.plane = plane;
+        a.hx = (T)(cfg.hx / S); a.hy = (T)cfg.hy; a.hz = (T)cfg.hz;
+        a.q2m = (T)cfg.plasma_q2m;
+        a.djx0 = (T)cfg.plasma_djx0; a.djy0 = (T)cfg.plasma_djy0; a.djz0 = (T)cfg.plasma_djz0;
+        a.drho0 = (T)cfg.plasma_drho0;
+        a.bxe = (T)cfg.bx_ext; a.bye = (T)cfg.by_ext; a.bze = (T)cfg.bz_ext;
+        a.sE = (T)(cfg.plasma_q2m * (cfg.hx / S) / 2.0);
+        a.hxhy = (T)((cfg.hx / S) / cfg.hy);
+        a.hxhz = (T)((cfg.hx / S) / cfg.hz);
+        a.invMy = 1.0f / (float)My;
+        a.lgMy = lg_my();
+        a.err = d_err;
+        return a;
+    }
+
     qs_status push(int iLayer, int iSplit, int full) override {
         (void)iLayer; (void)iSplit;
         // the fields and the plasma this push reads: with the averaged fields
@@ -1542,36 +1562,18 @@ struct Engine : EngineBase {
             qs_status s = cic_prepare();
             if (s) return s;
         }
-        PushArgs<T> a{};
-        a.n = np;
-        a.My = My; a.Mz = Mz;
+        PushArgs<T> a = push_args();
         a.cell = pcell;
         a.y = py; a.z = pz; a.px = ppx; a.py = ppy; a.pz = ppz; a.w = pw;
         a.P = from_avg ? Cf : Pf;   // (C + C) / 2 = C exactly
         a.C = Cf;
-        if (push_fields) {   // the adjoint's recomputation: the stored gathered fields
-            a.P = a.C = push_fields;
-            push_fields = nullptr;
-        }
         a.dep = Csrc;
         a.cell_out = pcell;
         a.dep_cell = nullptr;
-        a.plane = plane;
-        a.hx = (T)(cfg.hx / S); a.hy = (T)cfg.hy; a.hz = (T)cfg.hz;
-        a.q2m = (T)cfg.plasma_q2m;
-        a.djx0 = (T)cfg.plasma_djx0; a.djy0 = (T)cfg.plasma_djy0; a.djz0 = (T)cfg.plasma_djz0;
-        a.drho0 = (T)cfg.plasma_drho0;
-        a.bxe = (T)cfg.bx_ext; a.bye = (T)cfg.by_ext; a.bze = (T)cfg.bz_ext;
-        a.sE = (T)(cfg.plasma_q2m * (cfg.hx / S) / 2.0);
-        a.hxhy = (T)((cfg.hx / S) / cfg.hy);
-        a.hxhz = (T)((cfg.hx / S) / cfg.hz);
-        a.invMy = 1.0f / (float)My;
-        a.lgMy = lg_my();
         // lattice order (particle p seeded in cell p / ppc): the NGP
         // one-thread-per-cell kernel relies on it
         a.uniform_ppc = uniform_layout ? cfg.ppc : 0;
         a.full = full;
-        a.err = d_err;
         a.skip_dens = clear_by_maps() ? 1 : 0;   // the march never reads the density deposit
         a.favg = push_favg;
         push_favg = nullptr;
@@ -2344,7 +2346,7 @@ struct Engine : EngineBase {
             return fail(QS_ERR_UNSUPPORTED, "the adjoint needs 6 ny nz and 3 x the particle count "
                                             "below 2^31");
         CK(cudaStreamSynchronize(st));
-        void* old[] = {ck, seg, lam, lam_pm, lam_sb, d_dloss, ck_off, ck_cell, ck_id, seg_cell,
+        void* old[] = {ck, seg, lam, lam_pm, lam_sb, d_dloss, ck_cell, ck_id, seg_cell,
                        lam_pos, adj_inv, adj_tmp, fstore};
         for (void* p : old)
             if (p) cudaFree(p);
@@ -2375,9 +2377,10 @@ struct Engine : EngineBase {
             if ((s = alloc(&seg_cell, (size_t)K * np, "adjoint segment"))) return s;
             if ((s = alloc(&lam_pos, 2 * (size_t)np, "adjoint positions"))) return s;
             if (cic_sort) {
-                if ((s = alloc(&ck_id, (size_t)ck_count * np, "adjoint checkpoints"))) return s;
-                if ((s = alloc(&ck_off, (size_t)ck_count * off_stride(), "adjoint checkpoints")))
+                if ((s = alloc(&ck_id, (size_t)ck_count * (np + off_stride()),
+                               "adjoint checkpoints")))
                     return s;
+                ck_off = ck_id + (size_t)ck_count * np;   // behind the ids
                 if ((s = alloc(&adj_inv, (size_t)np, "adjoint reorder"))) return s;
                 if ((s = alloc(&adj_tmp, 5 * (size_t)np, "adjoint reorder"))) return s;
             }
@@ -2451,24 +2454,37 @@ struct Engine : EngineBase {
         klaunch(KC_MISC, [&] { return launch_save_state<T>(sc, st); });
     }
 
+    // the particles (and cells) entering layer i of the segment of checkpoint m
+    // that starts at layer c: in the checkpoint itself or the segment's slot
+    const T* entry_state(int m, int c, int i) const {
+        return i == c ? ck + (size_t)m * ck_stride() : seg + (size_t)(c - i) * seg_stride();
+    }
+    const int32_t* entry_cell(int m, int c, int i) const {
+        return i == c ? ck_cell + (size_t)m * np : seg_cell + (size_t)(c - i) * np;
+    }
+
     // with the field store: recompute the particles entering layers c .. lo
-    // of one segment from its checkpoint by the full pushes alone, each
-    // gathering the fields the march stored for it (its deposit is not read)
+    // of one segment from its checkpoint by the moves of the full pushes
+    // alone, each gathering the fields the march stored for it, from slot to
+    // slot
     qs_status recompute_states(int m, int c, int lo) {
-        in_march = true;
-        adj_recompute = true;
-        qs_status s = restore_checkpoint(m);
-        for (int i = c; !s && i >= lo; i--) {
-            save_entry(seg + (size_t)(c - i) * seg_stride(), i, c);
-            if (i > lo) {
-                push_fields = fstore_at(i, nIter);
-                s = push(i, 0, 1);
-            }
+        for (int i = c; i > lo; i--) {
+            PushArgs<T> a = push_args();
+            T* in = const_cast<T*>(entry_state(m, c, i));
+            T* out = seg + (size_t)(c - i + 1) * seg_stride();
+            a.full = 1;
+            a.move_only = 1;
+            a.cell = entry_cell(m, c, i);
+            a.y = in; a.z = in + np; a.px = in + 2 * np; a.py = in + 3 * np; a.pz = in + 4 * np;
+            a.P = a.C = fstore_at(i, nIter);
+            a.loff = cic_loff;   // (a grouped push)
+            a.y_out = out; a.z_out = out + np; a.px_out = out + 2 * np; a.py_out = out + 3 * np;
+            a.pz_out = out + 4 * np;
+            a.cell_out = seg_cell + (size_t)(c - i + 1) * np;
+            klaunch(KC_PUSH, [&] { return launch_push<T>(a, cfg.shape, sizeof(T) == 4, st); });
         }
-        push_fields = nullptr;
-        in_march = false;
-        adj_recompute = false;
-        return s;
+        CK(cudaGetLastError());
+        return QS_OK;
     }
 
     // recompute the layers c .. lo of one segment from its checkpoint, storing
@@ -2550,7 +2566,8 @@ struct Engine : EngineBase {
         a.cell = cic_adj ? slot_cell : pcell;   // NGP: the seeded cells never change
         a.lamPos = lam_pos;
         a.y = slot; a.z = slot + np; a.px = slot + 2 * np; a.py = slot + 3 * np;
-        a.pz = slot + 4 * np; a.w = pw;
+        a.pz = slot + 4 * np; a.w = adj_w;
+        a.early = (g_pdl && (fftx || fftx64)) ? 1 : 0;
         a.F = fields;
         a.lamD = lamp(LAM_D);
         a.lamPm = lam_pm;
@@ -2768,12 +2785,19 @@ struct Engine : EngineBase {
                 const bool stored = fstored(end);   // then every layer of the segment
                 qs_status s = stored ? recompute_states(m, c, end) : recompute_segment(m, c, end);
                 if (s) return s;
+                // the weights in this checkpoint's particle order
+                adj_w = stored ? ck + (size_t)m * ck_stride() + 5 * (size_t)np : pw;
                 side_adj = !prof && !fp32_study && adj_fused();
                 adj_pred_pending = false;
                 for (int i = end; i <= c && !s; i++) {
-                    const int32_t* sc = cic_adj ? seg_cell + (size_t)(c - i) * np : nullptr;
                     const T* slot = seg + (size_t)(c - i) * seg_stride();
-                    s = adjoint_layer(i, slot, sc, stored ? fstore_at(i, 0) : slot + 5 * (size_t)np);
+                    if (stored)
+                        s = adjoint_layer(i, entry_state(m, c, i), entry_cell(m, c, i),
+                                          fstore_at(i, 0));
+                    else
+                        s = adjoint_layer(i, slot,
+                                          cic_adj ? seg_cell + (size_t)(c - i) * np : nullptr,
+                                          slot + 5 * (size_t)np);
                 }
                 join_sides();   // the next recomputation rewrites what the sweep reads
                 side_adj = adj_pred_pending = false;

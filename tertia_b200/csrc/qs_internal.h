@@ -256,6 +256,10 @@ struct PushAdjArgs {
     size_t plane;
     T sE, hxhy, hxhz, djx0, djy0, djz0, bxe, bye, bze;
     int full, precise;
+    // CIC, 1: all inputs but lamD were complete before the kernel in front of
+    // this one in the launch chain started (its wait comes before lamD's first
+    // read; the recomputation of the push runs ahead of it)
+    int early;
     float invMy;          // 1 / My (cell -> (j, k) without an integer division)
 };
 template <class T>
