@@ -1198,7 +1198,6 @@ struct Engine : EngineBase {
         explicit PdlScope(bool on) { g_pdl = g_pdl || on; }
         ~PdlScope() { g_pdl = old; }
     };
-    bool dense_passes() const { return !tcx && !fftx && !fftx64; }
     bool chain_fft() const { return (fftx || fftx64) && use_pdl && !prof && !fp32_study; }
 
     qs_status beam_spectra() {
@@ -1579,12 +1578,11 @@ struct Engine : EngineBase {
         a.favg = push_favg;
         push_favg = nullptr;
         bool regroup = false;
-        // In the march a pass of the transforms that every thread of the
-        // kernel enters behind its wait (not so the tensor-core passes)
-        // stands between two pushes; a regrouping on the side stream may end
-        // only just before this push.
-        a.early = (g_pdl && in_march && !adj_recompute && (fft_maps() || dense_passes()) &&
-                   as_grouped && !after_regroup) ? 1 : 0;
+        // In the march a pass of the transforms stands between two pushes
+        // and every block of it triggers behind its own wait; a regrouping on
+        // the side stream may end only just before this push.
+        a.early = (g_pdl && in_march && !adj_recompute && !fp32_study && as_grouped &&
+                   !after_regroup) ? 1 : 0;
         if (cic_sort) {
             a.loff = cic_loff;
             a.bpref = cic_bpref;

@@ -243,16 +243,31 @@ __global__ void __launch_bounds__(THREADS_V2, 1)
     fence_after();
     const uint32_t tmem = tmem_slot;
     volatile int* abortp = &abort_flag;
-    qs::pdl_wait();   // operands and outputs are the previous kernel's
+    const int rowM = kind * p.K + n0;
+    const int rowD = f * p.R + m0;
+    auto load_matrix = [&](int kb) {   // and announce the whole stage
+        const uint32_t fb = smem_u32(&full_bar[kb % STAGES]);
+        mbar_expect_tx(fb, STAGE);
+        uint8_t* st = smem + (size_t)(kb % STAGES) * STAGE;
+#pragma unroll
+        for (int t = 0; t < NSPLIT; t++)
+            tma_load_2d(smem_u32(st + t * M_TILE), &mapM, fb, kb * BK, t * p.mat_rows + rowM);
+    };
+    // The matrix does not depend on the kernel in front: the first stages'
+    // tiles are fetched ahead of the wait (at 512^2 a block's k loop is eight
+    // steps, so a fetch from L2 at its head shows: a BF16x3 layer of eight
+    // passes 149.2 -> 147.6 us).
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapM) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapD) : "memory");
+        for (int kb = 0; kb < STAGES && kb < nkb; kb++) load_matrix(kb);
+    }
+    qs::pdl_wait();   // the data operand and the outputs are the previous kernel's
 
     if (warp == 0) {
         if (lane != 0) qs::pdl_trigger();
         if (lane == 0) {
             // ---------------- TMA producer
-            asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapM) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&mapD) : "memory");
-            const int rowM = kind * p.K + n0;
-            const int rowD = f * p.R + m0;
             int issued = 0;
             for (int kb = 0; kb < nkb; kb++) {
                 const int s = kb % STAGES;
@@ -262,13 +277,9 @@ __global__ void __launch_bounds__(THREADS_V2, 1)
                     *abortp = 1;
                     break;
                 }
+                if (kb >= STAGES) load_matrix(kb);
                 const uint32_t fb = smem_u32(&full_bar[s]);
-                mbar_expect_tx(fb, STAGE);
                 uint8_t* st = smem + (size_t)s * STAGE;
-#pragma unroll
-                for (int t = 0; t < NSPLIT; t++)
-                    tma_load_2d(smem_u32(st + t * M_TILE), &mapM, fb, kb * BK,
-                                t * p.mat_rows + rowM);
 #pragma unroll
                 for (int t = 0; t < NSPLIT; t++)
                     tma_load_2d(smem_u32(st + NSPLIT * M_TILE + t * D_TILE), &mapD, fb, kb * BK,
