@@ -445,7 +445,7 @@ def fp64_compare(cfg, beam, pushes_per_step, ours_ms):
     out = {"value": pushes_per_step / (r64["ms"] / 1e3), "unit": UNIT,
            "ms_per_step": r64["ms"],
            "speedup": r64["ms"] / ours_ms,
-           "transforms": "dense FP64 SIMT matrix passes (O(N^3) per plane)",
+           "transforms": "dense FP64 matrix passes on the FP64 tensor cores (O(N^3) per plane)",
            "fft": {"value": pushes_per_step / (r64f["ms"] / 1e3), "unit": UNIT,
                    "ms_per_step": r64f["ms"],
                    "speedup_over_fp64_plain": r64["ms"] / r64f["ms"],

@@ -5,12 +5,12 @@
 // at 512^2 with thermal spread nearly every particle has left its seeded cell
 // by the tail of the box.  The CIC push stages each cell tile's fields and
 // deposits in shared memory and pushes the particles of the tile, so the
-// particle arrays are regrouped by cell after each full push: a counting sort
+// particle arrays are regrouped by cell after every few full pushes: a counting sort
 // whose histogram the full push itself builds (atomic count per new cell), an
 // exclusive scan of the counts in one kernel (per 1024-cell block; the last
 // block to finish scans the block totals), and a scatter whose within-cell
 // rank is an atomic decrement of the count (so the counts end at zero, ready
-// for the next full push).  Each particle carries its load-order id so that
+// for the next counting push).  Each particle carries its load-order id so that
 // the host gets the plasma back in load order.
 #include "qs_common.cuh"
 #include "qs_internal.h"
