@@ -248,9 +248,9 @@ __global__ void __launch_bounds__(256) push_adjoint_kernel(PushAdjArgs<T> a) {
         a.lamPm[a.n + i] = bp[1];
         a.lamPm[2 * a.n + i] = bp[2];
     } else {
-        a.lamPm[i] += bp[0];
-        a.lamPm[a.n + i] += bp[1];
-        a.lamPm[2 * a.n + i] += bp[2];
+        atomicAdd(a.lamPm + i, bp[0]);
+        atomicAdd(a.lamPm + a.n + i, bp[1]);
+        atomicAdd(a.lamPm + 2 * a.n + i, bp[2]);
     }
     // fields: E = (P + C)/2 and B = (P + C)/2 + external
 #pragma unroll
@@ -580,11 +580,14 @@ __device__ __forceinline__ int push_adjoint_cic_one(const PushAdjArgs<T>& a, uin
         a.lamPos[i] = lyp;
         a.lamPos[un + i] = lzp;
     } else {
-        a.lamPm[i] += bp[0];
-        a.lamPm[un + i] += bp[1];
-        a.lamPm[2 * un + i] += bp[2];
-        a.lamPos[i] += lyp;
-        a.lamPos[un + i] += lzp;
+        // no one else adds to them: reductions only so that nothing waits for
+        // their values at the end of the thread (adjoint per layer, 256^2
+        // 65.4 -> 64.2 us, 512^2 195.4 -> 185.6, 1024^2 746 -> 703)
+        atomicAdd(a.lamPm + i, bp[0]);
+        atomicAdd(a.lamPm + un + i, bp[1]);
+        atomicAdd(a.lamPm + 2 * un + i, bp[2]);
+        atomicAdd(a.lamPos + i, lyp);
+        atomicAdd(a.lamPos + un + i, lzp);
     }
     return cell;
 }
