@@ -1,13 +1,18 @@
 // pdl.cuh — programmatic dependent launch for the kernels of the xi-march.
 //
-// A march is a long chain of dependent kernels (about 17 per layer), each
-// short (5-12 us).  Launched with the programmatic-stream-serialisation
+// A march is a long chain of dependent kernels (about 10 per layer), each
+// short (2-27 us).  Launched with the programmatic-stream-serialisation
 // attribute, a kernel may be scheduled before its predecessor has finished:
 // its prologue (barrier set-up, TMEM allocation, descriptor prefetch, index
 // math) overlaps the predecessor's tail, and pdl_wait() then blocks until the
 // predecessor has completed and its memory is visible.  Every kernel launched
 // through launch_pdl() calls pdl_wait() before it touches memory that an
 // earlier kernel writes or reads, so the ordering is that of a plain stream.
+// The exception are reads of data that were complete before the kernel in
+// front started: every block of that kernel triggers behind its own wait, so
+// whatever the kernel before it wrote is visible by then.  (Not so what a
+// kernel on a joined side stream wrote: it may have triggered before its
+// stores.)
 // pdl_trigger() lets the successor be scheduled; every thread of the kernel
 // calls it once its own share of the main work is issued.  Without the
 // attribute both instructions are no-ops.
