@@ -600,14 +600,18 @@ __device__ __forceinline__ void cic_substep(T dy, T dz, T ps, T& ytmp, T& ztmp, 
     wc[3] = ry * rz;
 }
 
-// Element i of an array.  In FP32 by a 32-bit byte offset from its base: one
-// address operand for all arrays of a particle or all planes of a node,
-// 95.3 -> 93.2 us per layer of the warm 512 x 512 march (the launch checks that
-// the arrays are below 4 GB).  In FP64, whose registers are full, the plain
-// form (180.7 us against 183.9).
-template <class T, class U>
-__device__ __forceinline__ U* at32(U* base, std::conditional_t<sizeof(T) == 4, unsigned, size_t> i) {
-    if constexpr (sizeof(T) == 4) {
+// Element i of an array.  In FP32 by a 32-bit byte offset from its base (Off =
+// unsigned): one address operand for all arrays of a particle or all planes of
+// a node, 95.3 -> 93.2 us per layer of the warm 512 x 512 march.  In FP64, whose
+// registers are full, the plain form (180.7 us against 183.9), and so for FP32
+// arrays of 4 GB and more (WIDE, chosen by the launch), which a byte offset
+// does not reach.
+template <class T, bool WIDE>
+using RowOff = std::conditional_t<sizeof(T) == 4 && !WIDE, unsigned, size_t>;
+template <class Off, class U>
+__device__ __forceinline__ U* at32(U* base, Off i) {
+    if constexpr (sizeof(Off) == 4) {
+        static_assert(sizeof(U) == 4);
         using B = std::conditional_t<std::is_const_v<U>, const char, char>;
         return reinterpret_cast<U*>(reinterpret_cast<B*>(base) + i * 4u);
     } else {
@@ -752,7 +756,7 @@ __device__ __forceinline__ PushStep<T> push_step(const PushArgs<T>& a, const T (
     return u;
 }
 
-template <int TY, int ND, int WIN, bool P2, class T>
+template <int TY, int ND, int WIN, bool P2, class T, bool WIDE = false>
 __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     using M = RowMath<T>;
     using FP = FPair<T>;
@@ -768,7 +772,7 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     __shared__ int Kl[TY][WIN + WIN / 32];       // counting push: the final cells
     const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
     const int My = a.My, Mz = a.Mz;
-    using Off = std::conditional_t<sizeof(T) == 4, unsigned, size_t>;
+    using Off = RowOff<T, WIDE>;
     const Off plane = (Off)a.plane;
     const int tiles_x = My / TX;
     const int j0 = (blockIdx.x % tiles_x) * TX, k0 = (blockIdx.x / tiles_x) * TY;
@@ -790,9 +794,9 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     T nx_y = zero, nx_z = zero, nx_px = zero, nx_py = zero, nx_pz = zero, nx_w = zero;
     if (pbeg + lane < pend) {
         const Off q = pbeg + lane;
-        nx_cell = *at32<T>(a.cell, q); nx_y = *at32<T>(a.y, q); nx_z = *at32<T>(a.z, q);
-        nx_px = *at32<T>(a.px, q); nx_py = *at32<T>(a.py, q); nx_pz = *at32<T>(a.pz, q);
-        nx_w = *at32<T>(a.w, q);
+        nx_cell = *at32<Off>(a.cell, q); nx_y = *at32<Off>(a.y, q); nx_z = *at32<Off>(a.z, q);
+        nx_px = *at32<Off>(a.px, q); nx_py = *at32<Off>(a.py, q); nx_pz = *at32<Off>(a.pz, q);
+        nx_w = *at32<Off>(a.w, q);
     }
     if (a.early) pdl_wait();
     QS_TRACE_WAITED();
@@ -804,15 +808,15 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
             if (one_set) {
 #pragma unroll
                 for (int q = 0; q < 3; q++)
-                    Fs[q][r][cc] = FP::make(ld(at32<T>(a.C + 2 * q * plane, m)),
-                                            ld(at32<T>(a.C + (2 * q + 1) * plane, m)));
+                    Fs[q][r][cc] = FP::make(ld(at32<Off>(a.C + 2 * q * plane, m)),
+                                            ld(at32<Off>(a.C + (2 * q + 1) * plane, m)));
             } else {
 #pragma unroll
                 for (int q = 0; q < 3; q++) {
-                    const P2T pp = FP::make(ld(at32<T>(a.P + 2 * q * plane, m)),
-                                            ld(at32<T>(a.P + (2 * q + 1) * plane, m)));
-                    const P2T cp = FP::make(ld(at32<T>(a.C + 2 * q * plane, m)),
-                                            ld(at32<T>(a.C + (2 * q + 1) * plane, m)));
+                    const P2T pp = FP::make(ld(at32<Off>(a.P + 2 * q * plane, m)),
+                                            ld(at32<Off>(a.P + (2 * q + 1) * plane, m)));
+                    const P2T cp = FP::make(ld(at32<Off>(a.C + 2 * q * plane, m)),
+                                            ld(at32<Off>(a.C + (2 * q + 1) * plane, m)));
                     Fs[q][r][cc] = FP::mul(half, FP::add(pp, cp));
                 }
             }
@@ -851,7 +855,7 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
         for (int d = 0; d < ND; d++) {
             const T x = q[d] * dj[d];
 #pragma unroll
-            for (int r = 0; r < 4; r++) atomicAdd(at32<T>(a.dep + d * plane, nd[r]), x * wc[r]);
+            for (int r = 0; r < 4; r++) atomicAdd(at32<Off>(a.dep + d * plane, nd[r]), x * wc[r]);
         }
     };
     for (int wbase = pbeg; wbase < pend; wbase += WIN) {
@@ -864,9 +868,9 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
             T px = nx_px, py = nx_py, pz = nx_pz;
             if (p + 32 < pend) {
                 const Off q = p + 32;
-                nx_cell = *at32<T>(a.cell, q); nx_y = *at32<T>(a.y, q); nx_z = *at32<T>(a.z, q);
-                nx_px = *at32<T>(a.px, q); nx_py = *at32<T>(a.py, q); nx_pz = *at32<T>(a.pz, q);
-                nx_w = *at32<T>(a.w, q);
+                nx_cell = *at32<Off>(a.cell, q); nx_y = *at32<Off>(a.y, q); nx_z = *at32<Off>(a.z, q);
+                nx_px = *at32<Off>(a.px, q); nx_py = *at32<Off>(a.py, q); nx_pz = *at32<Off>(a.pz, q);
+                nx_w = *at32<Off>(a.w, q);
             }
             int key = -1, last = cell;
             T qv[ND], ay = zero, az = zero;
@@ -907,8 +911,8 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                             T s = zero;
 #pragma unroll
                             for (int r = 0; r < 4; r++)
-                                s += wg[r] * half * (ld(at32<T>(a.P + f * plane, nn[r])) +
-                                                     ld(at32<T>(a.C + f * plane, nn[r])));
+                                s += wg[r] * half * (ld(at32<Off>(a.P + f * plane, nn[r])) +
+                                                     ld(at32<Off>(a.C + f * plane, nn[r])));
                             g[f] = s;
                         }
                     }
@@ -940,9 +944,9 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
                     last = jb + My * kb;
                     if (a.full) {
                         const Off q = p;
-                        *at32<T>(a.y, q) = ytmp; *at32<T>(a.z, q) = ztmp; *at32<T>(a.px, q) = px;
-                        *at32<T>(a.py, q) = py; *at32<T>(a.pz, q) = pz;
-                        *at32<T>(a.cell_out, q) = last;
+                        *at32<Off>(a.y, q) = ytmp; *at32<Off>(a.z, q) = ztmp; *at32<Off>(a.px, q) = px;
+                        *at32<Off>(a.py, q) = py; *at32<Off>(a.pz, q) = pz;
+                        *at32<Off>(a.cell_out, q) = last;
                     }
                 }
             }
@@ -1029,7 +1033,7 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
 #pragma unroll
         for (int d = 0; d < ND; d++) {
             const T x = Tt[d][fr][fc];
-            if (x != zero) atomicAdd(at32<T>(a.dep + d * plane, m), dj[d] * x);
+            if (x != zero) atomicAdd(at32<Off>(a.dep + d * plane, m), dj[d] * x);
         }
         fc += (32 * TY) % W;
         fr += (32 * TY) / W;
@@ -1111,10 +1115,17 @@ int launch_push_rows(const PushArgs<T>& a, cudaStream_t st) {
     constexpr int TY = 4, WIN = 128;
     if (a.move_only) return launch_move(a, st);
     if (!a.loff || a.dep_cell) return 0;   // grouped by cell with offsets (the engine checks the shape)
-    // 32-bit byte offsets into the particle arrays and the planes
-    if ((uint64_t)a.n * sizeof(T) >= (1ull << 32) || (uint64_t)a.plane * sizeof(T) >= (1ull << 32)) return 0;
     const dim3 grid((a.My / 32) * (a.Mz / TY));
     const dim3 block(32 * TY);
+    // FP32's 32-bit byte offsets reach arrays below 4 GB
+    if constexpr (sizeof(T) == 4)
+        if ((uint64_t)a.n >= (1ull << 30) || (uint64_t)a.plane >= (1ull << 30)) {
+            if (a.skip_dens)
+                launch_pdl(push_cic_row_kernel<TY, 3, WIN, false, T, true>, grid, block, 0, st, a);
+            else
+                launch_pdl(push_cic_row_kernel<TY, 4, WIN, false, T, true>, grid, block, 0, st, a);
+            return 1;
+        }
     if (a.skip_dens) {
         if (a.lgMy >= 0) launch_pdl(push_cic_row_kernel<TY, 3, WIN, true, T>, grid, block, 0, st, a);
         else launch_pdl(push_cic_row_kernel<TY, 3, WIN, false, T>, grid, block, 0, st, a);
