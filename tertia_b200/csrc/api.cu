@@ -1369,6 +1369,7 @@ struct Engine : EngineBase {
         Psrc = srcbuf;
         Csrc = srcbuf + 4 * plane;
         CK(cudaMemsetAsync(srcbuf, 0, 8 * plane * sizeof(T), st));
+        dens_clear[0] = dens_clear[1] = true;
         cur = 0;
         p_valid = true;
         if (front_layer) {
@@ -1376,6 +1377,7 @@ struct Engine : EngineBase {
             // forward transforms of its planes, as Guess computes them (:717-743)
             CK(cudaMemcpyAsync(Psrc, front_src, 4 * plane * sizeof(T), cudaMemcpyDeviceToDevice,
                                st));
+            dens_clear[0] = false;
             p_valid = false;
         }
         Pf = f3layer(L);
@@ -1440,7 +1442,7 @@ struct Engine : EngineBase {
             // predictor and the inverse y-pass of E, B in one kernel, then the z-pass
             SpecArgs<T> a = spec_args(iLayer, iSplit);
             a.zero_src = clear_by_maps() ? Csrc : nullptr;
-            a.skip_dens = (clear_by_maps() && cic_sort) ? 1 : 0;
+            a.skip_dens = density_clear(a.zero_src);
             a.lean = in_march ? 1 : 0;
             a.write_b = 0;
             // beside a pending last z-pass of the previous layer (reading
@@ -1522,6 +1524,18 @@ struct Engine : EngineBase {
     // Inside the march (no source store) the deposit planes are cleared by
     // the spectral kernel that precedes each push instead of by a memset.
     bool clear_by_maps() const { return in_march && !src3; }
+
+    // Whether a map that clears the deposit planes `bank` may leave the density
+    // out.  The grouped push adds none to it in the march, so once cleared (by
+    // the march's start, or by the first map that clears this bank) it stays so.
+    bool dens_clear[2] = {false, false};
+    int density_clear(const T* bank) {
+        if (!bank || !cic_sort) return 0;
+        bool& c = dens_clear[bank != srcbuf];
+        const int was = c;
+        c = true;
+        return was;
+    }
 
     // the sizes and the physics of a push
     PushArgs<T> push_args() {
@@ -1667,7 +1681,7 @@ struct Engine : EngineBase {
                 SpecArgs<T> a = spec_args(iLayer, iSplit);
                 a.write_b = 0;
                 a.zero_src = (clear_by_maps() && iter >= 0) ? Csrc : nullptr;
-                a.skip_dens = (clear_by_maps() && cic_sort) ? 1 : 0;
+                a.skip_dens = density_clear(a.zero_src);
                 a.lean = (in_march && iter >= 0) ? 1 : 0;
                 charge_args(a, iLayer, iSplit, iter);
                 const int nout = want_rho ? 7 : 6;
@@ -1680,7 +1694,7 @@ struct Engine : EngineBase {
                     an = spec_args(iLayer - 1, 0);
                     cur ^= 1;
                     an.zero_src = clear_by_maps() ? Psrc : nullptr;   // the next push's deposit
-                    an.skip_dens = a.skip_dens;
+                    an.skip_dens = density_clear(an.zero_src);
                     an.lean = 1;
                     an.write_b = 0;
                 }
@@ -2500,6 +2514,7 @@ struct Engine : EngineBase {
         pred_next = -1;
         next_avg = half_avg = false;
         fuse_lo = lo;
+        dens_clear[0] = dens_clear[1] = false;   // whatever was called since the march
         qs_status s = restore_checkpoint(m);
         for (int i = c; !s && i >= lo; i--) {
             T* slot = seg + (size_t)(c - i) * seg_stride();

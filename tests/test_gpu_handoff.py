@@ -127,6 +127,30 @@ def test_march_from_a_received_layer_matches_oracle(oracle_lib, prec, shape, gra
         h.close()
 
 
+@pytest.mark.parametrize("prec", ["fp64fft", "fp32"])
+@pytest.mark.parametrize("layers,n", [(2, 32), (2, 64), (12, 64)])
+def test_received_density_is_not_left_behind(prec, layers, n):
+    """The march clears both banks of sources before its pushes, the received
+    layer's density among them (the march itself keeps no density)."""
+    from tertia_b200.mesh import Mesh
+    full, half, beam, upper, empty = boxes(prec, abi.QS_SHAPE_CIC, n=n)
+    with Mesh(half) as up:
+        up.load_beam(upper)
+        up.load_front_plasma(wl.front_plasma(half, seed=5))
+        up.step()
+        buf = up.pack_layer()
+    assert np.max(np.abs(layout(buf, half)[0][9])) > 1e-3
+    low = half.copy()
+    low.nx = layers
+    with Mesh(low) as m:
+        m.load_beam(empty)
+        for _ in range(2):   # captured, then replayed
+            m.unpack_layer(buf)
+            m.step()
+            for bank in (abi.QS_LAYER_P, abi.QS_LAYER_C):
+                assert np.all(m.get_layer(bank, abi.QS_F_DENS) == 0), bank
+
+
 def test_two_boxes_equal_one_box():
     from tertia_b200.mesh import Mesh
     full, half, beam, upper, empty = boxes("fp64", abi.QS_SHAPE_NGP)
