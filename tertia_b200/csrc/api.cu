@@ -2284,6 +2284,10 @@ struct Engine : EngineBase {
     qs_status save_checkpoint(int m) {
         if (m >= ck_count || np != adj_np) return fail(QS_ERR_STATE, "checkpoint storage");
         join_sides();   // the regrouped plasma
+        // a regrouping that is still due comes first: the offsets kept below
+        // belong to the order of the particles kept here
+        if (cic_adj && cic_sort)
+            if (qs_status s = cic_prepare()) return s;
         T* dst = ck + (size_t)m * ck_stride();
         for (int c = 0; c < 5; c++)
             CK(cudaMemcpyAsync(dst + (size_t)c * np, particle_arrays(c), np * sizeof(T),
@@ -2304,7 +2308,6 @@ struct Engine : EngineBase {
                                    cudaMemcpyDeviceToDevice, st));
                 // the offsets of this order, whose grouping may be some pushes
                 // old (offsets counted from the current cells would not fit it)
-                if (qs_status s = cic_prepare()) return s;
                 int* off = ck_off + (size_t)m * off_stride();
                 CK(cudaMemcpyAsync(off, cic_loff, plane * sizeof(int), cudaMemcpyDeviceToDevice,
                                    st));
