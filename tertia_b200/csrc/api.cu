@@ -2345,6 +2345,8 @@ struct Engine : EngineBase {
                                    st));
                 CK(cudaMemcpyAsync(cic_bpref, off + plane, (off_stride() - plane) * sizeof(int),
                                    cudaMemcpyDeviceToDevice, st));
+                // (a counting push before may have left its histogram)
+                CK(cudaMemsetAsync(cic_cnt, 0, plane * sizeof(int), st));
                 grp.grouped = true;
                 grp.off_valid = true;
                 grp.counted = false;
