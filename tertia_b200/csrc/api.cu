@@ -1683,6 +1683,9 @@ struct Engine : EngineBase {
                 a.zero_src = (clear_by_maps() && iter >= 0) ? Csrc : nullptr;
                 a.skip_dens = density_clear(a.zero_src);
                 a.lean = (in_march && iter >= 0) ? 1 : 0;
+                // since the last kernel that wrote its bank (a map) a z-pass, a
+                // push and the deposit's z-pass have run
+                a.early = in_march ? 1 : 0;
                 charge_args(a, iLayer, iSplit, iter);
                 const int nout = want_rho ? 7 : 6;
                 // the layer's last corrector also runs the next layer's

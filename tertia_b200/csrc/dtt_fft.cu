@@ -842,11 +842,13 @@ __host__ __device__ constexpr int spec_threads() {
 // What bounds it: the latency of its serial phases (load, y-pass of J, map,
 // inverse y-pass), with four CTAs per SM at ny = 512, more than its traffic.
 // The ten rows the corrector reads (the P bank, the density before, the beam)
-// were complete before the z-pass in front of this kernel started, so they
-// are fetched by cp.async ahead of the wait and land during the y-pass of J,
-// in shared memory that is free until the map: the E, B, Rho rows (the thread
-// that reads a mode pair overwrites it) and the work space of the idle
-// groups.  Of its outputs only those that something reads are stored
+// are fetched by cp.async ahead of the wait and land during the y-pass of J.
+// The caller says that they were complete before the kernel in front started
+// (SpecArgs::early: in the march a push and a z-pass stand in between); else
+// the launch leaves the chain and the kernel starts behind the one in front.
+// They land in shared memory that is free until the map: the E, B, Rho rows
+// (the thread that reads a mode pair overwrites it) and the work space of the
+// idle groups.  Of its outputs only those that something reads are stored
 // (SpecArgs::lean).  Against loads in the map, 4 + 3 more planes stored per
 // layer and the predictor's P bank read back from memory: layer of the warm
 // 512 x 512 x 1024 march 96.9 -> 94.4-95.4 us, 1024 x 1024 390 -> 384 us, FP64
@@ -1083,10 +1085,12 @@ cudaError_t launch_spec_rows(const SpecArgs<typename Cx<C>::Real>& a,
                              const SpecArgs<typename Cx<C>::Real>* next, cudaStream_t st) {
     const dim3 grid((unsigned)a.nz), block(spec_threads<M, C>());
     const size_t sm = spec_rows_smem<M, C>();
+    // the correctors fetch rows ahead of their wait
+    const bool chain = g_pdl && a.early;
     if (next)
-        return launch_pdl(spec_rows_fn<M, true, true, C>(), grid, block, sm, st, a, r, *next);
+        return launch_ex(chain, spec_rows_fn<M, true, true, C>(), grid, block, sm, st, a, r, *next);
     if (correct)
-        return launch_pdl(spec_rows_fn<M, true, false, C>(), grid, block, sm, st, a, r, a);
+        return launch_ex(chain, spec_rows_fn<M, true, false, C>(), grid, block, sm, st, a, r, a);
     return launch_pdl(spec_rows_fn<M, false, false, C>(), grid, block, sm, st, a, r, a);
 }
 

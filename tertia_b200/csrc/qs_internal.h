@@ -41,6 +41,11 @@ struct SpecArgs {
     // alone; the layer's last corrector (lean 0) stores the bank the next
     // layer reads.
     int lean;
+    // 1 (the same kernels, correctors): the P bank, Rho and the beam spectra
+    // were complete before the kernel in front of this one in the launch chain
+    // started (they are read ahead of the wait for it; 0: launched outside the
+    // chain)
+    int early;
     // optional (correctors): FP64 charge sums (charge.cuh); each block writes
     // its partial sums of rho c_ky c_kz and Jx c_ky c_kz to qsum[2 * block]
     double* qsum;
