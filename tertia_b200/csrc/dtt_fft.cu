@@ -380,18 +380,26 @@ __device__ __forceinline__ void cp_async16(void* s, const void* g) {
                  : "memory");
 }
 
+// p[r * ld + c] by a 32-bit byte offset (a plane is 16 MB at most): half the
+// address arithmetic of the 2 V loads a thread issues
+template <class Real>
+__device__ __forceinline__ Real at_row(const Real* p, int r, int ld, int c) {
+    const unsigned off = ((unsigned)r * (unsigned)ld + (unsigned)c) * (unsigned)sizeof(Real);
+    return *reinterpret_cast<const Real*>(reinterpret_cast<const char*>(p) + off);
+}
+
 // Whether the column transform brings its tile to shared memory by cp.async
 // (else every thread loads its own values into registers).  Both are bound by
 // latency, about 10 to 20 warps per SM of one load, two or three exchanges
-// and one store.  Staging takes half the registers (62 against 158 at M = 512,
-// where the direct form leaves one CTA on an SM) but adds a trip through
-// shared memory and a barrier.  Layers of a march: 1024 x 1024 382 us direct,
-// 349 us staged; 256 x 256 41.8 and 40.7 us; 512 x 512 95.3 us direct, 96.4 us
-// (8 values per thread) and 98.7 us (16) staged, FP64 180.5 and 183.7 us;
-// the adjoint's accumulating passes at 256 x 256 86.2 and 87.2 us.
-template <int M, bool ACC, class C>
+// and one store.  Staging takes fewer registers (FP32 72 against 128 at M =
+// 512, FP64 64 against 96) but adds a trip through shared memory and a
+// barrier.  Layers of a march, direct / staged: FP32 64 x 64 25.6 / 25.9 us,
+// 128 x 128 30.0 / 30.3, 256 x 256 38.3 / 38.5, 512 x 512 90.9 / 94.7,
+// 1024 x 1024 343 / 332, 512 x 2048 320 / 324; FP64 256 x 256 50.7 / 53.1,
+// 512 x 512 176.5 / 180.5, 1024 x 1024 739 / 706.
+template <int M>
 __host__ __device__ constexpr bool cols_staged() {
-    return M >= 512 || (M == 128 && !ACC && sizeof(C) == sizeof(float2));
+    return M >= 512;
 }
 
 // The adjoint's extra of a column pass: the input values a thread holds are
@@ -426,11 +434,30 @@ __device__ __forceinline__ void add_and_clear(const Real (&lo)[V], const Real (&
     }
 }
 
+// Blocks per SM the direct column kernel is compiled for.  Left to itself (0)
+// ptxas spares registers, 40 to 64, by spacing the loads out between the
+// arithmetic that uses them, and each load's latency shows: the kernel is a
+// few warps per SM of 2 V loads, exchanges and stores.  With one block asked
+// for it takes 80 (FP32) and 96 (FP64) and issues the loads at once.  FP32 of
+// 16 values per thread (n = 512) does best with six (80 registers), which
+// also leaves room for blocks of the next kernel in the chain: 512 x 512 x 1024
+// march 91.8 us per layer for one block, 91.1 for six, 90.9 for five, but
+// transforms of 6 and 64 planes 11.2 / 96 us for one, 11.1 / 105 for six,
+// 11.6 / 106 for five.  Per layer, left to itself and so: 64 x 64 28.3 -> 25.9
+// us, 128 x 128 32.3 -> 30.0, 512 x 512 x 128 84.2 -> 79.9, FP64 512 x 512
+// 177.8 -> 176.5.  The adjoint's form, which adds and clears behind the loads,
+// does best left to itself (adjoint per layer at 512 x 512 168.5 us, 172 with
+// one block asked for).
+template <int M, bool ACC, class C>
+__host__ __device__ constexpr int cols_min_blocks() {
+    return ACC ? 0 : vpt_c<M, C>() > 8 ? 6 : 1;
+}
+
 // Transform along the strided axis: a CTA takes TJ adjacent columns of one
 // plane (TJ floats = whole 32-byte sectors per row); column c's sequence
 // lives at W[e * TJ + c], its T threads are TJ lanes apart.
 template <int M, int TJ, class C, int NF = kMaxXfFields, bool ACC = false>
-__global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()))
+__global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()), cols_min_blocks<M, ACC, C>())
     fft_cols_kernel(ColArgsT<typename Cx<C>::Real, NF> a) {
     using Real = typename Cx<C>::Real;
     constexpr int V = vpt_c<M, C>();
@@ -468,30 +495,11 @@ __global__ void __launch_bounds__(TJ * (M / vpt_c<M, C>()))
 #pragma unroll
     for (int b = 0; b < V; b++) {
         const int i = jt + bitrev<V>(b) * T;
-        lo[b] = inf[(size_t)(2 * i) * ld + col];
-        hi[b] = inf[(size_t)(2 * M - 1 - 2 * i) * ld + col];
+        lo[b] = at_row(inf, 2 * i, a.ncols, col);
+        hi[b] = at_row(inf, 2 * M - 1 - 2 * i, a.ncols, col);
         w[b] = __ldg(pre + i);
     }
-    if constexpr (ACC) {
-        add_and_clear<V, T, M>(lo, hi, accf, clrf, jt, col, ld);
-    } else if (accf || clrf) {
-        // never taken, but with it compiled in all loads are issued before any
-        // arithmetic (72 registers and slower without it)
-#pragma unroll
-        for (int b = 0; b < V; b++) {
-            const int i = jt + bitrev<V>(b) * T;
-            const size_t olo = (size_t)(2 * i) * ld + col;
-            const size_t ohi = (size_t)(2 * M - 1 - 2 * i) * ld + col;
-            if (accf) {
-                accf[olo] += lo[b];
-                accf[ohi] += hi[b];
-            }
-            if (clrf) {
-                clrf[olo] = Real(0);
-                clrf[ohi] = Real(0);
-            }
-        }
-    }
+    if constexpr (ACC) add_and_clear<V, T, M>(lo, hi, accf, clrf, jt, col, ld);
     C v[V];
 #pragma unroll
     for (int b = 0; b < V; b++) {
@@ -641,17 +649,17 @@ __host__ __device__ constexpr int cols_tj() {
     return (M / vpt_c<M, C>()) >= 16 ? 8 : (M / vpt_c<M, C>()) >= 4 ? 16 : 32;
 }
 
-template <int M, bool ACC, class C = float2>
+template <int M, class C = float2>
 size_t cols_smem() {
     // the tables, and the work space or the padded input tile in its place
     return sizeof(C) * (size_t)M * 2 + sizeof(typename Cx<C>::Real) * (size_t)cols_tj<M, C>() *
-                                           (2 * M + (cols_staged<M, ACC, C>() ? M / 2 : 0));
+                                           (2 * M + (cols_staged<M>() ? M / 2 : 0));
 }
 
 // the column kernel of a launch (ACC: with planes to add to or to clear)
 template <int M, bool ACC, class C>
 constexpr auto cols_fn() {
-    if constexpr (cols_staged<M, ACC, C>()) return fft_cols_staged_kernel<M, cols_tj<M, C>(), ACC, C>;
+    if constexpr (cols_staged<M>()) return fft_cols_staged_kernel<M, cols_tj<M, C>(), ACC, C>;
     else return fft_cols_kernel<M, cols_tj<M, C>(), C, kMaxXfFields, ACC>;
 }
 
@@ -659,13 +667,13 @@ template <int M, class C = float2>
 cudaError_t set_cols_smem() {
     const cudaError_t e = cudaFuncSetAttribute(cols_fn<M, false, C>(),
                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)cols_smem<M, false, C>());
+                                               (int)cols_smem<M, C>());
     if (e != cudaSuccess) return e;
     if constexpr (sizeof(C) != sizeof(float2)) return e;   // the adjoint's passes are FP32
     else
         return cudaFuncSetAttribute(cols_fn<M, true, C>(),
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)cols_smem<M, true, C>());
+                                    (int)cols_smem<M, C>());
 }
 
 template <int M, class C = float2>
@@ -682,8 +690,8 @@ cudaError_t launch_cols(const ColArgsT<typename Cx<C>::Real>& a, int nf, cudaStr
     const dim3 grid((unsigned)(a.ncols / TJ), (unsigned)nf), block(TJ * (M / vpt_c<M, C>()));
     if constexpr (sizeof(C) == sizeof(float2))
         if (a.acc[0] || a.clr[0])   // the adjoint's passes
-            return launch_pdl(cols_fn<M, true, C>(), grid, block, cols_smem<M, true, C>(), st, a);
-    return launch_pdl(cols_fn<M, false, C>(), grid, block, cols_smem<M, false, C>(), st, a);
+            return launch_pdl(cols_fn<M, true, C>(), grid, block, cols_smem<M, C>(), st, a);
+    return launch_pdl(cols_fn<M, false, C>(), grid, block, cols_smem<M, C>(), st, a);
 }
 
 // The z-passes of two layers' E, B in one launch (12 planes), up to nz = 256
