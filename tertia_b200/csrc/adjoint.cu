@@ -833,7 +833,7 @@ __global__ void __launch_bounds__(256) beam_weight_grad_kernel(BeamGradArgs<T> a
                                Vx * (double)a.lb3[(l * 2 + 1) * plane + m]);
                 }
     }
-    a.out[p] = g * a.polarity;
+    a.out[p] = scalbn(g * a.polarity, -(int)*a.shift);
 }
 
 template <class T>

@@ -357,7 +357,8 @@ struct Engine : EngineBase {
     T* lam_sb = nullptr;        // layers lam_lo..nx x 2 planes: adjoint of the beam spectra, then
                                 // (in place) of the real beam currents
     int lam_lo = -1;            // first layer lam_sb holds (the lowest one a sweep reaches)
-    T* d_dloss = nullptr;       // nx: d loss / d on-axis Ex of each layer
+    // nx: d loss / d on-axis Ex of each layer, times 2^k; then k (adjoint())
+    T* d_dloss = nullptr;
     double* d_gradw = nullptr;  // nb: d loss / d beam weight
     // CIC adjoint: checkpointed cells and ids, the cells entering each layer of
     // a segment, the position adjoint, and the reorder between checkpoints
@@ -2392,7 +2393,7 @@ struct Engine : EngineBase {
         if ((s = alloc(&seg, (size_t)K * seg_stride(), "adjoint segment"))) return s;
         if ((s = alloc(&lam, (size_t)LAM_N * plane, "adjoint planes"))) return s;
         if ((s = alloc(&lam_pm, 3 * (size_t)np, "adjoint momenta"))) return s;
-        if ((s = alloc(&d_dloss, (size_t)L, "loss gradient"))) return s;
+        if ((s = alloc(&d_dloss, (size_t)L + 1, "loss gradient"))) return s;
         cic_adj = cfg.shape == QS_SHAPE_CIC;
         if (cic_adj) {
             if ((s = alloc(&ck_cell, (size_t)ck_count * np, "adjoint checkpoints"))) return s;
@@ -2842,6 +2843,7 @@ struct Engine : EngineBase {
         g.lb3 = lam_sb;
         g.plane = plane;
         g.polarity = cfg.beam_polarity;
+        g.shift = d_dloss + L;
         g.out = d_gradw;
         klaunch(KC_BEAM_PUSH, [&] { return launch_beam_weight_grad<T>(g, st); });
         CK(cudaGetLastError());
@@ -2884,9 +2886,21 @@ struct Engine : EngineBase {
             }
         }
         {
-            std::vector<T> h(L);
-            for (int i = 0; i < L; i++) h[i] = (T)dloss[i];
-            CK(cudaMemcpyAsync(d_dloss, h.data(), L * sizeof(T), cudaMemcpyHostToDevice, st));
+            // FP32: the sweep's sums are reductions in memory, which flush
+            // subnormal values.  The adjoint is linear, so it runs on the loss
+            // gradient times 2^k and the result is scaled back: the largest
+            // entry at 2^40 puts what is flushed below what FP32 would resolve
+            // without the scaling, and leaves 2^87 for the sweep to grow.
+            double top = 0.0;
+            for (int i = 0; i < L; i++) top = std::max(top, std::fabs(dloss[i]));
+            int k = 0;
+            if (sizeof(T) == 4 && top > 0.0 && std::isfinite(top))
+                k = std::max(0, 40 - std::ilogb(top));
+            std::vector<T> h(L + 1);
+            for (int i = 0; i < L; i++) h[i] = (T)std::ldexp(dloss[i], k);
+            h[L] = (T)k;
+            CK(cudaMemcpyAsync(d_dloss, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice,
+                               st));
             CK(cudaStreamSynchronize(st));
         }
         if (cfg.use_graph && !prof) {

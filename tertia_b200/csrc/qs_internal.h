@@ -394,6 +394,7 @@ struct BeamGradArgs {
     const T* lb3;
     size_t plane;
     double polarity;
+    const T* shift;    // the adjoints are 2^*shift times what they stand for
     double* out;
 };
 template <class T>

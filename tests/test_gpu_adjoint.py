@@ -216,3 +216,23 @@ def test_wake_loss_with_bin_weights_on_the_gpu():
     with pytest.raises(RuntimeError, match="state is no longer"):
         l1.backward()
     m.close()
+
+
+@pytest.mark.parametrize("prec,n,shape", [("fp32", 32, QS_SHAPE_CIC), ("fp32", 64, QS_SHAPE_CIC),
+                                          ("fp32", 64, QS_SHAPE_NGP), ("fp64fft", 64, QS_SHAPE_CIC)])
+def test_adjoint_is_linear_down_to_small_loss_gradients(prec, n, shape):
+    """A loss in other units: the gradient scales with it, also where FP32
+    itself would hold its adjoints as subnormal numbers or not at all.  The
+    runs differ by the order of their atomic additions, as between checkpoint
+    intervals above."""
+    cfg, m, beam, bins, coeff = setup(prec, layers=24, n=n, shape=shape)
+    m.load_beam(beam)
+    m.move_beam_particles()
+    g = []
+    for s in (1.0, 1e-25, 1e-30, 1e-36, 1e-60, 1e12):
+        m.move_all_split_layers()
+        g.append(m.adjoint(coeff * s) / s)
+    m.close()
+    assert np.linalg.norm(g[0]) > 0
+    for q in g[1:]:
+        assert rel(q, g[0]) < 1e-5
