@@ -306,7 +306,10 @@ struct Engine : EngineBase {
     // march: its E, B in field-store layer nx, its sources and beam spectra here
     bool front_layer = false;
     bool front_used = false;    // a march has started from it (it serves one march)
-    bool graph_front = false;   // the captured march was built with a received front
+    // what the captured march was built for: a received front or the empty
+    // one, the number of particles and whether they lie in lattice order
+    bool graph_front = false, graph_uniform = false;
+    int64_t graph_np = -1;
     T* front_src = nullptr;     // Jx, Jy, Jz, Rho of the received layer
     T* front_beam = nullptr;    // RhoBeam, JxBeam spectra of the received layer
     // CIC in FP32, and in FP64 on FFT transforms, keeps the plasma grouped by
@@ -371,6 +374,7 @@ struct Engine : EngineBase {
     cudaGraphExec_t adj_exec = nullptr;   // captured sweep for the layers adj_lo .. head
     int adj_lo = -1;
     int64_t adj_graph_nb = -1;
+    bool adj_uniform = false;             // captured for particles in lattice order
     int64_t adj_kernels = 0;
     int64_t adj_np = 0, adj_nb = 0;
 
@@ -2235,12 +2239,15 @@ struct Engine : EngineBase {
             ck_valid = !s && ck_every > 0 && !front_layer;
             return s;
         }
-        if (gexec && graph_front != front_layer) {   // the head layer's set-up differs
+        if (gexec && (graph_front != front_layer || graph_np != np ||
+                      graph_uniform != uniform_layout)) {
             cudaGraphExecDestroy(gexec);
             gexec = nullptr;
         }
         if (!gexec) {
             graph_front = front_layer;
+            graph_np = np;
+            graph_uniform = uniform_layout;
             cudaGraph_t g = nullptr;
             CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             capturing = g_capturing = true;
@@ -2870,7 +2877,8 @@ struct Engine : EngineBase {
             adj_nb = nb;
             drop_adjoint_graph();
         }
-        if (nb != adj_graph_nb) drop_adjoint_graph();   // the beam count is baked in
+        // the beam count and the particles' layout are baked in
+        if (nb != adj_graph_nb || adj_uniform != uniform_layout) drop_adjoint_graph();
         {
             // the beam-spectrum adjoint covers the layers the sweep reaches
             // (from the lowest layer with a nonzero loss entry to the head)
@@ -2930,6 +2938,7 @@ struct Engine : EngineBase {
                 }
                 adj_lo = lo;
                 adj_graph_nb = nb;
+                adj_uniform = uniform_layout;
                 adj_kernels = capture_count;
                 adj_end = HostState{Pf, Cf, Psrc, Csrc, cur, grp};
             }
