@@ -2234,7 +2234,12 @@ struct Engine : EngineBase {
             qs_status s = beam_spectra();
             if (s) return s;
         }
-        if (!cfg.use_graph || prof) {
+        // Single pushes since the front was loaded may have regrouped the
+        // plasma into the other set, or left a regrouping due; the captured
+        // march starts from a fresh front in the first set.
+        const bool fresh = !cic_sort || (!grp.flip && grp.grouped && !grp.off_valid &&
+                                         !grp.counted && grp.since == 0);
+        if (!cfg.use_graph || prof || !fresh) {
             qs_status s = march_device();
             ck_valid = !s && ck_every > 0 && !front_layer;
             return s;

@@ -784,8 +784,10 @@ __global__ void __launch_bounds__(32 * TY) push_cic_row_kernel(PushArgs<T> a) {
     // In the march nothing since the kernel before last writes them, so they
     // need not wait for the kernel in front either.
     if (!a.early) pdl_wait();
-    const int lo = cell_offset(a, mycell);
-    const int hi = (Off)(mycell + 1) < plane ? cell_offset(a, mycell + 1) : (int)a.n;
+    // (offsets out of step with the arrays, which the regrouping reports, stay
+    // inside them)
+    const int lo = min(cell_offset(a, mycell), (int)a.n);
+    const int hi = (Off)(mycell + 1) < plane ? min(cell_offset(a, mycell + 1), (int)a.n) : (int)a.n;
     for (int i = threadIdx.x; i < ND * H * W; i += 32 * TY) (&Tt[0][0][0])[i] = zero;
     const int pbeg = __shfl_sync(0xffffffffu, lo, 0);
     const int pend = __shfl_sync(0xffffffffu, hi, 31);

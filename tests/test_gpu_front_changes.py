@@ -1,5 +1,6 @@
 """A handle whose march was captured, then given another front: another number
-of particles or another layout of the same number.  The march by graph equals the march launch by launch."""
+of particles, another layout of the same number, or single pushes between the
+front and the march.  The march by graph equals the march launch by launch."""
 import numpy as np
 import pytest
 
@@ -34,8 +35,10 @@ def marches(cfg, graph, every=0):
     with Mesh(cfg) as m:
         m.load_beam(wl.small_beam(cfg, n=2000))
         m.move_beam_particles()
-        for front in (a, b, c, a):
+        for front, pushes in ((a, 0), (b, 0), (c, 0), (a, 1), (b, 2), (c, 4), (a, 5), (a, 0)):
             m.load_front_plasma(front)
+            for _ in range(pushes):
+                m.move_particles_layer(0, 0, 1)
             m.move_all_split_layers()
             m.sync()
             out.append((m.onaxis_ex(), m.get_field3d(QS_F_EY, 1), m.get_plasma()["w"]))
