@@ -2281,6 +2281,8 @@ struct Engine : EngineBase {
         cur = graph_end.cur;
         if (graph_end.grp.flip != grp.flip) swap_sets();
         grp = graph_end.grp;
+        cur_layer = 0;   // where the march ended (qs_get_layer's beam currents)
+        cur_split = S - 1;
         p_valid = true;
         marched = true;
         tail_ready = true;

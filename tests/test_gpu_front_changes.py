@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from tertia_b200 import workload as wl
-from tertia_b200.abi import QS_F_EY, QS_SHAPE_CIC, QS_SHAPE_NGP
+from tertia_b200.abi import (QS_F_EY, QS_F_RHOBEAM, QS_LAYER_C, QS_SHAPE_CIC, QS_SHAPE_NGP)
 from gpu_helpers import cfg_for, rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -83,3 +83,20 @@ def test_captured_adjoint_with_another_layout(monkeypatch, store):
     for x, y in zip(grads[:2], grads[2:]):
         assert np.linalg.norm(x) > 0
         assert rel_l2(y, x) < 1e-4
+
+
+def test_layer_after_a_replayed_march():
+    """After a march by graph the C layer is layer 0, whichever layer single
+    calls stopped at before."""
+    from tertia_b200.mesh import Mesh
+    cfg = cfg_for("fp64", n=32, layers=6, shape=QS_SHAPE_NGP, ts=0.0, synchrotron=0)
+    with Mesh(cfg) as m:
+        m.load_beam(wl.small_beam(cfg, n=2000))
+        m.move_beam_particles()
+        m.move_all_split_layers()
+        first = m.get_layer(QS_LAYER_C, QS_F_RHOBEAM)
+        m.begin_march()
+        m.layer_begin(cfg.nx - 2, 0)
+        assert np.any(m.get_layer(QS_LAYER_C, QS_F_RHOBEAM) != first)
+        m.move_all_split_layers()
+        np.testing.assert_array_equal(m.get_layer(QS_LAYER_C, QS_F_RHOBEAM), first)
