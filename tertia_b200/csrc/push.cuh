@@ -1151,9 +1151,12 @@ int launch_push(const PushArgs<T>& a, int shape, bool precise, cudaStream_t st) 
     if (shape == QS_SHAPE_NGP) {
         if constexpr (F32) {
             if (a.uniform_ppc == 4 && a.n == (int64_t)a.My * a.Mz * 4 && !a.dep_cell) {
-                // small grids: one warp per block spreads the cells over the SMs
-                const int cells = a.My * a.Mz, nt = cells >= 148 * 128 ? 128 : 32;
-                launch_pdl(push_cell_kernel<4>, dim3((cells + nt - 1) / nt), dim3(nt), 0, st, a);
+                // blocks of one warp, to spread a small grid's cells over the
+                // SMs, are no better there (march per layer at 64 x 64 20.7 us
+                // against 20.5, 128 x 128 23.6 against 23.0) and worse from
+                // 128 x 256 on (27.2 against 26.2)
+                const int cells = a.My * a.Mz;
+                launch_pdl(push_cell_kernel<4>, dim3((cells + 127) / 128), dim3(128), 0, st, a);
                 return 1;
             }
             launch_pdl(push_kernel<T, QS_SHAPE_NGP, true, true>, dim3(blocks), dim3(threads), 0, st, a);
