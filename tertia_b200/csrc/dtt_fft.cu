@@ -1038,9 +1038,8 @@ __device__ __forceinline__ void spectral_rows_body(SpecArgs<typename Cx<C>::Real
 }
 
 // Two CTAs per SM where the shared memory of two fits: on the 1024-wide FP32
-// grid (M = 512: 512 threads at most 64 registers; 84 KB each, 108 KB with the
-// next predictor) and on the 512-wide FP64 grid (256 threads at most 128
-// registers; 86 KB, 110 KB).
+// grid (M = 512: 512 threads at most 64 registers; 84 KB each) and on the
+// 512-wide FP64 grid (256 threads at most 128 registers; 86 KB).
 template <int M, bool CORRECT, bool PRED_NEXT, class C = float2>
 __global__ void __launch_bounds__(spec_threads<M, C>(),
                                   (M == 512 || (M == 256 && sizeof(C) == sizeof(double2))) ? 2 : 1)

@@ -45,9 +45,8 @@ __device__ __forceinline__ double one_minus_vx(double px, double py, double pz, 
     return px > 0.0 ? fwd : bwd;
 }
 
-// Approximate reciprocal square root: PTX rsqrt.approx.ftz.f32, the same
-// instruction rsqrtf uses without the rescaling of subnormal arguments (the
-// arguments here are 1 + p^2).
+// Approximate reciprocal square root, PTX rsqrt.approx.ftz.f32 (subnormal
+// arguments count as zero; the arguments here are 1 + p^2).
 __device__ __forceinline__ float rsq_approx(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

@@ -139,7 +139,8 @@ struct DttFft {
     bool spec_rows = false;    // run_spectral_rows available (ny in [64, 1024])
     bool planes = false;       // run_planes available (ny, nz in 32, 64, 128)
     static DttFft* create(int ny, int nz);   // nullptr when a size is not handled
-    // both passes in one launch, a plane per CTA; 0 when the job does not fit it
+    // both passes in one launch, a cluster of 1 to 4 CTAs per plane; 0 when the
+    // job does not fit it
     int run_planes(const DttJob<float>& job, cudaStream_t st) const;
     int run_pass(int pass, const DttJob<float>& job, float* scratch, cudaStream_t st) const;
     // the z-pass alone: nf planes in -> out, y-spectral or real alike; with
@@ -177,7 +178,8 @@ struct DttFft64 {
     double2* tab_y = nullptr;
     double2* tab_z = nullptr;
     bool spec_rows = false;    // run_spectral_rows available (ny in [64, 512])
-    bool planes = false;       // run_planes available (ny, nz in 32, 64, 128)
+    // run_planes available (ny, nz in 32, 64, 128; at most 8192 values)
+    bool planes = false;
     static DttFft64* create(int ny, int nz);   // nullptr when a size is not handled
     int run_planes(const DttJob<double>& job, cudaStream_t st) const;
     int run_pass(int pass, const DttJob<double>& job, double* scratch, cudaStream_t st) const;
