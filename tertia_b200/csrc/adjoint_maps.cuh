@@ -18,33 +18,6 @@ __device__ __forceinline__ void add_to(T* p, T v) { atomicAdd(p, v); }
 __device__ __forceinline__ void add_to(float* p, float w, float v) { atomicAdd(p, w * v); }
 __device__ __forceinline__ void add_to(double* p, double w, double v) { *p = fma(w, v, *p); }
 
-// A divisor of several of a mode's terms.  FP32 multiplies by its reciprocal:
-// the gradient's error against 64 bits (256 x 256, 10 seeds, 4 runs each) is
-// 4.9e-7 in the geometric mean, 5.8e-7 with divisions, and the adjoint takes
-// 60.3 us per layer, 61.2 with them (1024 x 1024 624 and 630).  FP64 divides.
-template <class T>
-struct Divisor;
-template <>
-struct Divisor<float> {
-    float r;
-    __device__ __forceinline__ explicit Divisor(float x) : r(1.f / x) {}
-};
-template <>
-struct Divisor<double> {
-    double x;
-    __device__ __forceinline__ explicit Divisor(double d) : x(d) {}
-};
-__device__ __forceinline__ float operator/(float a, Divisor<float> d) { return a * d.r; }
-__device__ __forceinline__ double operator/(double a, Divisor<double> d) { return a / d.x; }
-__device__ __forceinline__ Divisor<float> operator*(Divisor<float> a, Divisor<float> b) {
-    a.r *= b.r;
-    return a;
-}
-__device__ __forceinline__ Divisor<double> operator*(Divisor<double> a, Divisor<double> b) {
-    a.x *= b.x;
-    return a;
-}
-
 template <class T>
 __device__ __forceinline__ void beam_adj(const AdjSpecArgs<T>& a, size_t n, T lrb, T lrbp,
                                          T ljxb) {
@@ -69,6 +42,11 @@ __device__ __forceinline__ void put_lp(const AdjSpecArgs<T>& a, int f, size_t n,
     else add_to(a.lP[f] + n, v);
 }
 
+// The divisions below stay divisions: products with the reciprocals of k2,
+// d + k2 and the denominator save 0.9 us of a 256 x 256 layer (60.4 against
+// 61.3), but the FP32 gradient's error against 64 bits is then 5 to 15% larger
+// on short boxes (512 x 512 x 58 layers 1.1e-7 against 0.96e-7).
+//
 // Transpose of corrector_kernel (IterateFieldsHydroLinLayerSplit's per-mode
 // update, movefieldshydrolinlayersplit.cpp:1419-1466) at mode (j, k): le, lb
 // are the adjoints of its spectral E, B outputs; lj gets the adjoint of its
@@ -81,20 +59,19 @@ __device__ __forceinline__ void corrector_adjoint_mode(const AdjSpecArgs<T>& a, 
     const T akz = a.piZ * (T(k) + T(0.5));
     const T aky = a.piY * (T(j) + T(0.5));
     const T k2 = aky * aky + akz * akz;
-    const Divisor<T> dk2(k2), ddk(d + k2);
     const T lrho = opt(a.lRho, n);
     const T lex = le[0] + opt(a.lEb[0], n);
     T ley = le[1] + opt(a.lEb[1], n);
     T lez = le[2] + opt(a.lEb[2], n);
     const T lbx = lb[0], lby = lb[1], lbz = lb[2];
     // by = (-akz (jx + jxb) + d ez)/k2, bz = (aky (jx + jxb) - d ey)/k2
-    lez += d * lby / dk2;
-    ley -= d * lbz / dk2;
-    const T ljxs = (-akz * lby + aky * lbz) / dk2;          // d(by,bz)/d(jx + jxb)
+    lez += d * lby / k2;
+    ley -= d * lbz / k2;
+    const T ljxs = (-akz * lby + aky * lbz) / k2;          // d(by,bz)/d(jx + jxb)
     T ljx = lrho + ljxs + opt(a.lJb[0], n);
-    T ljy = -hx * T(0.5) * aky * lrho - aky / dk2 * lex + akz / dk2 * lbx + opt(a.lJb[1], n);
-    T ljz = -hx * T(0.5) * akz * lrho - akz / dk2 * lex - aky / dk2 * lbx + opt(a.lJb[2], n);
-    const T lsrc = (aky * ley + akz * lez) / ddk;     // src = rb + rbp + rp + rho_old
+    T ljy = -hx * T(0.5) * aky * lrho - aky / k2 * lex + akz / k2 * lbx + opt(a.lJb[1], n);
+    T ljz = -hx * T(0.5) * akz * lrho - akz / k2 * lex - aky / k2 * lbx + opt(a.lJb[2], n);
+    const T lsrc = (aky * ley + akz * lez) / (d + k2);     // src = rb + rbp + rp + rho_old
     lj[0] = ljx;
     lj[1] = ljy;
     lj[2] = ljz;
@@ -121,18 +98,17 @@ __device__ __forceinline__ void predictor_adjoint_mode(const AdjSpecArgs<T>& a, 
     const T akz = a.piZ * (T(k) + T(0.5));
     const T aky = a.piY * (T(j) + T(0.5));
     const T k2 = aky * aky + akz * akz;
-    const Divisor<T> dk2(k2), ddk(d + k2);
-    const Divisor<T> den(T(4) + d * hx * hx);
+    const T den = T(4) + d * hx * hx;
     const T prop = (T(4) - d * hx * hx) / den;
     const T lrho = opt(a.lRho, n);
     T lex = le[0], ley = le[1], lez = le[2];
     const T lbx = lb[0], lby = lb[1], lbz = lb[2];
     // b from the predicted currents and fields
-    const T ljx = (-akz * lby + aky * lbz) / dk2;   // also the jxb adjoint
-    const T ljy = akz * lbx / dk2;
-    const T ljz = -aky * lbx / dk2;
-    lez += d * lby / dk2;
-    ley -= d * lbz / dk2;
+    const T ljx = (-akz * lby + aky * lbz) / k2;   // also the jxb adjoint
+    const T ljy = akz * lbx / k2;
+    const T ljz = -aky * lbx / k2;
+    lez += d * lby / k2;
+    ley -= d * lbz / k2;
     // jx = jxp + hx d (ex + exp)/2 (and y, z)
     const T hd2 = hx * d * T(0.5);
     lex += hd2 * ljx;
@@ -140,13 +116,13 @@ __device__ __forceinline__ void predictor_adjoint_mode(const AdjSpecArgs<T>& a, 
     lez += hd2 * ljz;
     T lexp = hd2 * ljx, leyp = hd2 * ljy, lezp = hd2 * ljz;
     // ey = -eyp + aky src/(d + k2), src = rb + rbp + rp + rho
-    const T lsrc = (aky * ley + akz * lez) / ddk;
+    const T lsrc = (aky * ley + akz * lez) / (d + k2);
     leyp -= ley;
     lezp -= lez;
     const T lrho_t = lrho + lsrc;
     // rho = prop rp - (rb + rbp) d hx^2/den + 4 exp hx (k2 + d)/den
     // ex  = prop exp - 2 (2 rp + rb + rbp) d hx / ((k2 + d) den)
-    const T cex = T(2) * d * hx / (ddk * den);
+    const T cex = T(2) * d * hx / ((k2 + d) * den);
     const T lrp = lsrc + prop * lrho_t - T(2) * cex * lex;
     const T lrb = lsrc - d * hx * hx / den * lrho_t - cex * lex;
     lexp += T(4) * hx * (k2 + d) / den * lrho_t + prop * lex;
