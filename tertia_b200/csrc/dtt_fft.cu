@@ -445,12 +445,12 @@ __device__ __forceinline__ void add_and_clear(const Real (&lo)[V], const Real (&
 // transforms of 6 and 64 planes 11.2 / 96 us for one, 11.1 / 105 for six,
 // 11.6 / 106 for five.  Per layer, left to itself and so: 64 x 64 28.3 -> 25.9
 // us, 128 x 128 32.3 -> 30.0, 512 x 512 x 128 84.2 -> 79.9, FP64 512 x 512
-// 177.8 -> 176.5.  The adjoint's form, which adds and clears behind the loads,
-// does best left to itself (adjoint per layer at 512 x 512 168.5 us, 172 with
-// one block asked for).
+// 177.8 -> 176.5, the adjoint at 256 x 256 61.0 -> 60.6.  The adjoint's form of
+// 16 values, which adds and clears behind the loads, does best left to itself
+// (adjoint per layer at 512 x 512 168.3 us, 172 with one block asked for).
 template <int M, bool ACC, class C>
 __host__ __device__ constexpr int cols_min_blocks() {
-    return ACC ? 0 : vpt_c<M, C>() > 8 ? 6 : 1;
+    return vpt_c<M, C>() <= 8 ? 1 : ACC ? 0 : 6;
 }
 
 // Transform along the strided axis: a CTA takes TJ adjacent columns of one
