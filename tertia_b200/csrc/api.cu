@@ -375,6 +375,7 @@ struct Engine : EngineBase {
     int adj_lo = -1;
     int64_t adj_graph_nb = -1;
     bool adj_uniform = false;             // captured for particles in lattice order
+    bool adj_restores = false;            // it restores checkpoints (into the plasma arrays)
     int64_t adj_kernels = 0;
     int64_t adj_np = 0, adj_nb = 0;
 
@@ -2365,13 +2366,18 @@ struct Engine : EngineBase {
                                    cudaMemcpyDeviceToDevice, st));
                 // (a counting push before may have left its histogram)
                 CK(cudaMemsetAsync(cic_cnt, 0, plane * sizeof(int), st));
-                grp.grouped = true;
-                grp.off_valid = true;
-                grp.counted = false;
-                grp.since = 0;
+                grouping_restored();
             }
         }
         return QS_OK;
+    }
+    // the plasma stands as a checkpoint left it, with that order's offsets
+    void grouping_restored() {
+        grp.grouped = true;
+        grp.off_valid = true;
+        grp.counted = false;
+        grp.since = 0;
+        adj_restores = true;
     }
 
     qs_status adjoint_checkpoints(int every) override {
@@ -2928,6 +2934,7 @@ struct Engine : EngineBase {
                 capturing = g_capturing = true;
                 capture_count = 0;
                 g_pdl = use_pdl;
+                adj_restores = false;
                 qs_status s = adjoint_device(lo);
                 g_pdl = false;
                 capturing = g_capturing = false;
@@ -2951,6 +2958,7 @@ struct Engine : EngineBase {
             }
             CK(cudaGraphLaunch(adj_exec, st));
             launches += adj_kernels;
+            if (adj_restores) grouping_restored();
             Pf = adj_end.Pf; Cf = adj_end.Cf; Psrc = adj_end.Psrc; Csrc = adj_end.Csrc;
             cur = adj_end.cur;
         } else {

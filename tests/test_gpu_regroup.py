@@ -88,3 +88,29 @@ def test_pushes_after_an_adjoint(monkeypatch, prec, profile):
         m.sync()
         np.testing.assert_array_equal(m.get_plasma()["w"],
                                       np.asarray(front["w"], np.float32 if prec == "fp32" else float))
+
+
+def test_pushes_after_a_replayed_adjoint(monkeypatch):
+    """The same when the sweep is replayed: single pushes leave a regrouping
+    due, and the replay restores checkpoints like the captured run did."""
+    from tertia_b200.mesh import Mesh
+    monkeypatch.setenv("QS_ADJ_FIELDS", "0")
+    cfg = wl.small_config(n=64, layers=8, ts=0.0, synchrotron=0, shape=QS_SHAPE_CIC)
+    cfg.precision = PRECISIONS["fp32"]
+    front = wl.front_plasma(cfg, seed=3)
+    g = np.zeros(cfg.nx)
+    g[:2] = 1.0
+    with Mesh(cfg) as m:
+        m.load_beam(wl.small_beam(cfg, n=2000))
+        m.load_front_plasma(front)
+        m.adjoint_checkpoints(4)
+        m.move_beam_particles()
+        for _ in range(3):
+            m.load_front_plasma(front)
+            m.move_all_split_layers()
+            for _ in range(4):
+                m.move_particles_layer(0, 0, 1)
+            assert np.any(m.adjoint(g))
+            for _ in range(5):
+                m.move_particles_layer(0, 0, 1)
+            m.sync()
